@@ -220,9 +220,12 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
         o_bmt = pk.vec(blk_bm_table(hp));
     }
     size_t o_ext = chy_mixed_pack_tables(&hp, &pk.host, precision == CHY_PREC_MIXED);
-    p->table_bytes = pk.host.size();
+    // tables formed on the device follow the packed image
+    const size_t o_dev = (pk.host.size() + 255) & ~(size_t)255;
+    const size_t nth = precision == CHY_PREC_FP64 ? thomas_table_doubles(hp.J, hp.K, hp.L) : 0;
+    p->table_bytes = o_dev + 2 * nth * sizeof(double);
     ce = cudaMalloc(&p->d_tables, p->table_bytes);
-    if (ce == cudaSuccess) ce = cudaMemcpy(p->d_tables, pk.host.data(), p->table_bytes, cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(p->d_tables, pk.host.data(), pk.host.size(), cudaMemcpyHostToDevice);
     if (ce != cudaSuccess) {
         chy_plan_destroy(p);
         return ce == cudaErrorMemoryAllocation ? fail(CHY_ERR_NOMEM, "tables") : cuda_fail(ce, "tables");
@@ -264,6 +267,17 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     t.an = (const double *)(D + o_an); t.bn = (const double *)(D + o_bn); t.cn = (const double *)(D + o_cn);
     t.U = (const double *)(D + o_U); t.V = (const double *)(D + o_V); t.lam = (const double *)(D + o_lam);
     for (int i = 0; i < 11; i++) t.zx[i] = hp.zx[i];
+    if (nth) {
+        double *rec = (double *)(D + o_dev), *mul = rec + nth;
+        t.th_rec = rec;
+        t.th_mul = mul;
+        ce = launch_thomas_table(t, rec, mul, cudaStreamLegacy);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(cudaStreamLegacy);
+        if (ce != cudaSuccess) {
+            chy_plan_destroy(p);
+            return cuda_fail(ce, "elimination table");
+        }
+    }
     if (precision == CHY_PREC_FP64_BLKTRI) {
         t.blk.nvec = bs.nvec;
         t.blk.nstage = (int)bs.stages.size();
@@ -282,7 +296,6 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     Work &w = p->w;
     w.sX = nX;
     w.sW = precision == CHY_PREC_FP64 ? nX : 0;
-    w.sC = precision == CHY_PREC_FP64 ? nX : 0;
     w.smom = (size_t)21 * hp.nring;
     w.ssub = nsub * 2 * hp.ncol;
     w.sscan = (nsub + 1) * 2 * hp.ncol;
@@ -293,7 +306,7 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     const bool blk = precision == CHY_PREC_FP64_BLKTRI;
     const size_t nbvec = blk ? al(blk_vector_doubles(t, max_batch)) : 0;
     const size_t nbscr = blk ? al(blk_scratch_doubles(t, max_batch, p->num_sms)) : 0;
-    const size_t per = al(w.sX * max_batch) + al(w.sW * max_batch) + al(w.sC * max_batch) +
+    const size_t per = al(w.sX * max_batch) + al(w.sW * max_batch) +
                        al(w.smom * max_batch) + al(w.ssub * max_batch) + al(w.sscan * max_batch) +
                        al(w.sphac * max_batch) + al(w.sdiag * max_batch) + nbvec + nbscr;
     size_t ext = chy_mixed_work_doubles(p);
@@ -306,7 +319,6 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     double *q = (double *)p->d_work;
     w.X = q; q += al(w.sX * max_batch);
     w.W = q; q += al(w.sW * max_batch);
-    w.C = q; q += al(w.sC * max_batch);
     w.mom = q; q += al(w.smom * max_batch);
     w.sub = q; q += al(w.ssub * max_batch);
     w.scan = q; q += al(w.sscan * max_batch);
@@ -504,7 +516,7 @@ long long chy_plan_bytes_per_solve(const chy_plan *p)
 {
     if (!p) return 0;
     const Work &w = p->w;
-    size_t per = w.sX + w.sW + w.sC + w.smom + w.ssub + w.sscan + w.sphac + w.sdiag;
+    size_t per = w.sX + w.sW + w.smom + w.ssub + w.sscan + w.sphac + w.sdiag;
     if (p->precision == CHY_PREC_FP64_BLKTRI) per += (size_t)p->t.blk.nvec * p->t.M * p->t.L;
     return (long long)(per * sizeof(double));
 }
@@ -1089,7 +1101,7 @@ extern "C" int chy_solve_static(chy_plan *p, const double *rho, double *phi, voi
     // the plan's per-solve arrays, 256-byte aligned pieces, carved from the static array
     const Work &pw = p->w;
     auto al = [](size_t n) { return (n + 31) & ~(size_t)31; };
-    const size_t need = al(pw.sX) + al(pw.sW) + al(pw.sC) + al(pw.smom) + al(pw.ssub) + al(pw.sscan) +
+    const size_t need = al(pw.sX) + 2 * al(pw.sW) + al(pw.smom) + al(pw.ssub) + al(pw.sscan) +
                         al(pw.sphac) + al(pw.sdiag);
     if (need * sizeof(double) > kStaticScratchBytes)
         return fail(CHY_ERR_CAPACITY, "chy_solve_static: this grid needs " + std::to_string(need * sizeof(double)) +
@@ -1120,7 +1132,6 @@ extern "C" int chy_solve_static(chy_plan *p, const double *rho, double *phi, voi
     double *q = base;
     w.X = q; q += al(pw.sX);
     w.W = q; q += al(pw.sW);
-    w.C = q; q += al(pw.sC);
     w.mom = q; q += al(pw.smom);
     w.sub = q; q += al(pw.ssub);
     w.scan = q; q += al(pw.sscan);

@@ -7,7 +7,6 @@
 //                          (the unknowns of the mode solve), j = J-1 the outer
 //                          boundary column, k = K-1 the top boundary row.
 //   W    [L][J][K]   FP64  vertical eigen coefficients of the mode solve
-//   C    [L][J][K]   FP64  radial elimination multipliers (FP64 solve path)
 //   MOM  [21][nring] FP64  per-ring azimuthal moments sum_l {1, cos m psi_l,
 //                          sin m psi_l} rho, ring = k*(J-1) + j.
 //   SUB  [nsub][2][ncol]   per sub-chunk sums of the boundary integrands.
@@ -82,6 +81,8 @@ struct DevTables {
     const double *am, *cm, *cc, *bm0, *xlamm, *an, *bn, *cn;
     // vertical eigenbasis, row-major [NZ][NZ]: U(p,k) and V(k,p)
     const double *U, *V, *lam;
+    // radial elimination table of the FP64 path, [N+1][M][K]: pivot reciprocals, multipliers
+    const double *th_rec, *th_mul;
     double zx[11];
     BlkDev blk;                     // CHY_PREC_FP64_BLKTRI plans only
 };
@@ -94,8 +95,8 @@ struct BatchPtrs {
 };
 
 struct Work {
-    double *X, *W, *C, *mom, *sub, *scan, *phac, *diag;
-    size_t sX, sW, sC, smom, ssub, sscan, sphac, sdiag;   // per-solve strides (elements)
+    double *X, *W, *mom, *sub, *scan, *phac, *diag;
+    size_t sX, sW, smom, ssub, sscan, sphac, sdiag;   // per-solve strides (elements)
     double *coef;                                    // optional /COEFS/ output (solve 0 only)
     double *bvec, *bscr;                             // BLKTRI-order path (k_blktri.cu)
 };
@@ -148,6 +149,9 @@ cudaError_t launch_forward(const DevTables &t, const BatchPtrs &bp, const Work &
 cudaError_t launch_bdy_sums(const DevTables &t, const Work &w, int nb, cudaStream_t s);
 cudaError_t launch_bdy_synth(const DevTables &t, const Work &w, int nb, cudaStream_t s);
 cudaError_t launch_solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s);
+// Doubles of each plane of the FP64 path's elimination table, and its kernel.
+size_t thomas_table_doubles(int J, int K, int L);
+cudaError_t launch_thomas_table(const DevTables &t, double *rec, double *mul, cudaStream_t s);
 // BLKTRI-order FP64 mode solves (k_blktri.cu): gather, cyclic reduction, scatter.
 // Stage schedule: nw warps per CTA (4, 8 or 16), up to ctas_per_sm CTAs per SM,
 // nw * ctas_per_sm <= 16.

@@ -13,194 +13,373 @@
 // This file holds the plain FP64 version of that pipeline.
 //
 // W layout: [l][j][p] (p fastest, leading dimension K) so the radial sweeps
-// of 32 consecutive p's read and write coalesced rows.
+// of 32 consecutive p's read and write coalesced rows.  Column p = K-1 holds
+// zero.
+//
+// The vertical transforms run on the FP64 tensor pipe (mma.sync m8n8k4, IEEE
+// fused multiply-adds like the scalar pipe's).  A CTA of sixteen warps keeps
+// the eigenbasis matrix in registers as mma fragments, eight of its rows per
+// warp, and walks (solve, l, j-tile) items through three shared-memory
+// buffers filled by asynchronous copies two tiles ahead, one barrier a tile.
+// At 8 solves of 256x128x256 (17.2 GFLOP each way, padded): forward 2.33 ->
+// 0.605 ms, inverse 2.43 -> 0.591 ms, 29 TFLOP/s, 78% of the FP64 tensor pipe
+// (ncu).  Before, scalar 4 x 4 register tiles read eight shared-memory values
+// per 16 multiply-adds (7.2 TFLOP/s).  Measured on the way: eight warps with 16
+// rows each 0.835 / 0.697 ms; m16n8k8 products in place of m8n8k4 the same as
+// these (0.665 / 0.659 ms against 0.661 / 0.642); 64-bit item divisions in
+// every warp cost 0.02-0.05 ms.
 #include "devplan.h"
 
 namespace chy {
 
-constexpr int kPB = 128;   // p / k extent held in shared memory (NZ <= 127)
-constexpr int kJT = 32;    // j columns per GEMM tile
+constexpr int kZThreads = 512;
+
+// Tile shape for KP = max(KMAX, 16): NWP warps along the 8-row blocks of the
+// eigenbasis, NWJ warps along j, 8 MT columns each.  Shared-memory rows are
+// padded so that the 16 lanes of a fragment load's half warp (4 x 4 elements)
+// fall on 16 different 8-byte banks: leading dimensions are 4 or 12 mod 16.
+template <int KP, int MT>
+struct ZTile {
+    static constexpr int NWP = KP / 8, NWJ = 16 / NWP, JT = 8 * MT * NWJ, KS = KP / 4;
+    static constexpr int LDY = JT + 4, LDW = KP + 4;
+    static constexpr int kFwdBuf = KP * LDY, kInvBuf = JT * LDW;   // doubles
+    static constexpr size_t kFwdBytes = (size_t)3 * kFwdBuf * 8, kInvBytes = (size_t)3 * kInvBuf * 8;
+};
+
+__device__ __forceinline__ void z_cp16(double *dst, const double *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void z_cp8(double *dst, const double *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void z_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void z_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 __device__ __forceinline__ int mode_m(int l, int n) { return l <= n ? l : l - n; }
 
-// Y(j,k) = 4 pi G Xhat(j,k) with the Dirichlet boundary folded in
-// (pot/pot3.f:212-224).
-__device__ __forceinline__ double rhs_value(const DevTables &t, const double *Xl, int j, int k)
+// c += a b, the warp-wide 8 x 8 x 4 FP64 product: a holds A[lane/4][lane%4],
+// b holds B[lane%4][lane/4], c holds C[lane/4][2 (lane%4) + {0, 1}].
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
 {
-    double y = t.pig4 * Xl[(size_t)k * t.J + j];
-    if (k == t.NZ - 1) y = y - t.cnmax * Xl[(size_t)t.NZ * t.J + j];
-    if (j == t.M - 1) y = y - t.cmmax * Xl[(size_t)k * t.J + t.M];
-    return y;
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
 }
 
-// W[l][j][p] = sum_k U(p,k) Y_l(j,k).  Persistent: each CTA keeps U in shared
-// memory and walks (batch, l, j-tile) items.
-__global__ void __launch_bounds__(256) k_zfwd_f64(DevTables t, Work w, int nb)
+// W[l][j][p] = sum_k U(p,k) Y_l(j,k), Y(j,k) = 4 pi G Xhat(j,k) with the
+// Dirichlet boundary folded in (pot/pot3.f:212-224).  The tile holds X as it
+// lies in memory, the boundary row k = NZ with it: 4 pi G is a factor of the
+// fragments, and row NZ's fragment -CN(NZ) U(p, NZ-1) folds the top boundary.
+// The outer boundary column is folded into column M-1 in shared memory.
+template <int KP, int MT>
+__global__ void __launch_bounds__(kZThreads, 1) k_zfwd_f64(DevTables t, Work w, int nb)
 {
-    extern __shared__ double smem[];
-    double *Us = smem;                  // [k][p], kPB x kPB
-    double *Ys = smem + kPB * kPB;      // [k][j], kPB x kJT
-    const int NZ = t.NZ, tid = threadIdx.x;
-    for (int i = tid; i < kPB * kPB; i += blockDim.x) {
-        const int k = i / kPB, p = i % kPB;
-        Us[i] = (k < NZ && p < NZ) ? t.U[(size_t)p * NZ + k] : 0.0;
+    using Z = ZTile<KP, MT>;
+    extern __shared__ __align__(16) double smem[];   // [3][KP][LDY]
+    const int NZ = t.NZ, M = t.M, J = t.J, K = t.K, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wp = warp % Z::NWP, wj = warp / Z::NWP;
+    double u[Z::KS];
+#pragma unroll
+    for (int s = 0; s < Z::KS; ++s) {
+        const int k = 4 * s + lane % 4, p = wp * 8 + lane / 4;
+        u[s] = (k < NZ && p < NZ) ? t.pig4 * t.U[(size_t)p * NZ + k]
+               : (k == NZ && p < NZ) ? -(t.cnmax * t.U[(size_t)p * NZ + NZ - 1]) : 0.0;
     }
-    const int njt = (t.M + kJT - 1) / kJT;
-    const long long items = (long long)nb * t.L * njt;
-    const int tp = tid / 8, tj = tid % 8, p0 = tp * 4, jj0 = tj * 4;
-    for (long long it = blockIdx.x; it < items; it += gridDim.x) {
-        const int jt = (int)(it % njt), l = (int)((it / njt) % t.L), b = (int)(it / ((long long)njt * t.L));
-        const int j0 = jt * kJT;
-        const double *Xl = w.X + (size_t)b * w.sX + (size_t)l * t.K * t.J;
-        __syncthreads();
-        for (int i = tid; i < NZ * kJT; i += blockDim.x) {
-            const int k = i / kJT, jj = i % kJT, j = j0 + jj;
-            Ys[k * kJT + jj] = (j < t.M) ? rhs_value(t, Xl, j, k) : 0.0;
+    // rows k >= K and columns no copy reaches start as zeros
+    for (int i = tid; i < 3 * Z::kFwdBuf; i += kZThreads) smem[i] = 0.0;
+    __syncthreads();
+    const int njt = (M + Z::JT - 1) / Z::JT;
+    const int items = nb * t.L * njt;   // item = (solve * L + mode) * njt + tile
+    const bool even = (J & 1) == 0;
+    const double edge = t.cmmax / t.pig4;
+    auto load = [&](int it, double *Y) {
+        if (it < items) {
+            const int q = it / njt, j0 = (it - q * njt) * Z::JT;
+            const double *Xl = w.X + (size_t)q * K * J;
+            const int nj = J - j0 < Z::JT ? J - j0 : Z::JT;
+            if (even) {
+                constexpr int H = Z::JT / 2;
+                for (int i = tid; i < K * H; i += kZThreads) {
+                    const int k = i / H, c = 2 * (i % H);
+                    if (c < nj) z_cp16(Y + k * Z::LDY + c, Xl + (size_t)k * J + j0 + c);
+                }
+            } else {
+                for (int i = tid; i < K * Z::JT; i += kZThreads) {
+                    const int k = i / Z::JT, c = i % Z::JT;
+                    if (c < nj) z_cp8(Y + k * Z::LDY + c, Xl + (size_t)k * J + j0 + c);
+                }
+            }
         }
+        z_commit();
+    };
+    int it = blockIdx.x;
+    load(it, smem);
+    load(it + (int)gridDim.x, smem + Z::kFwdBuf);
+    for (int buf = 0; it < items; it += gridDim.x, buf = buf == 2 ? 0 : buf + 1) {
+        double *Yt = smem + buf * Z::kFwdBuf;
+        z_wait<1>();
         __syncthreads();
-        double acc[4][4] = {};
-        for (int k = 0; k < NZ; ++k) {
-            double u[4], y[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) { u[a] = Us[k * kPB + p0 + a]; y[a] = Ys[k * kJT + jj0 + a]; }
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[a][c] = fma(u[a], y[c], acc[a][c]);
+        // every warp is past the previous tile: its buffer takes the tile after next
+        load(it + 2 * (int)gridDim.x, smem + (buf == 0 ? 2 : buf - 1) * Z::kFwdBuf);
+        const int q = it / njt, jt = it - q * njt;
+        if (jt == njt - 1) {
+            // Y(k, M-1) -= CM(M) X(k, M) for the tile's last column
+            const double *Xl = w.X + (size_t)q * K * J;
+            const int c = M - 1 - jt * Z::JT;
+            if (tid < NZ)
+                Yt[tid * Z::LDY + c] -= edge * (c + 1 < Z::JT ? Yt[tid * Z::LDY + c + 1] : Xl[(size_t)tid * J + M]);
+            __syncthreads();
         }
-        double *Wl = w.W + (size_t)b * w.sW + (size_t)l * t.J * t.K;
+        const double *Y = Yt + (lane % 4) * Z::LDY + wj * 8 * MT + lane / 4;
+        double acc[MT][2] = {};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int j = j0 + jj0 + c;
-            if (j < t.M)
+        for (int s = 0; s < Z::KS; ++s) {
+            double a[MT];
 #pragma unroll
-                for (int a = 0; a < 4; ++a)
-                    if (p0 + a < NZ) Wl[(size_t)j * t.K + p0 + a] = acc[a][c];
+            for (int m = 0; m < MT; ++m) a[m] = Y[4 * s * Z::LDY + 8 * m];
+#pragma unroll
+            for (int m = 0; m < MT; ++m) dmma(acc[m], a[m], u[s]);
+        }
+        double *Wl = w.W + (size_t)q * J * K;
+        const int p = wp * 8 + 2 * (lane % 4);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            const int j = jt * Z::JT + wj * 8 * MT + 8 * m + lane / 4;
+            if (j < M && p < K) *reinterpret_cast<double2 *>(Wl + (size_t)j * K + p) = make_double2(acc[m][0], acc[m][1]);
         }
     }
 }
 
-// Radial tridiagonal sweeps (T_r(m) + lam_p) w = W_p, one thread per (l, p).
-// BM_m(j) as pot/pot3.f:226-230 builds it.  Forward elimination stores the
-// multipliers in C (same layout as W), back substitution overwrites W.
-__global__ void __launch_bounds__(128) k_thomas_f64(DevTables t, Work w)
+// Elimination table of the radial systems (T_r(m) + lam_p): per (m, j, p) the
+// pivot reciprocal 1/d_j and the multiplier c_j/d_j, BM_m(j) as
+// pot/pot3.f:226-230 builds it.  They depend on the grid only, so a plan forms
+// them once; each of the L modes reads the slice of its m = mode_m(l).
+__global__ void __launch_bounds__(128) k_thomas_table(DevTables t, double *rec, double *mul)
 {
-    const int p = threadIdx.x, l = blockIdx.x, b = blockIdx.z;
+    const int p = threadIdx.x, m = blockIdx.x, M = t.M, K = t.K;
     if (p >= t.NZ) return;
-    const int m = mode_m(l, t.N), M = t.M, K = t.K;
     const double xl2 = 2.0 * (t.xlamm[m] - 1.0);
     const double axis = ((m % 2 == 0) ? 1.0 : -1.0) - 1.0;
     const double lam = t.lam[p];
-    double *__restrict__ Wp = w.W + (size_t)b * w.sW + (size_t)l * t.J * K + p;
-    double *__restrict__ Cp = w.C + (size_t)b * w.sC + (size_t)l * t.J * K + p;
-    constexpr int kU = 8;   // rows whose loads are issued ahead of the recurrence
-    double d = t.bm0[0] + axis * t.ammin + xl2 * t.cc[0] + lam;
-    double r = 1.0 / d;
-    double cprev = t.cm[0] * r, yprev = Wp[0] * r;
-    Cp[0] = cprev;
-    Wp[0] = yprev;
-    for (int j0 = 1; j0 < M; j0 += kU) {
-        double yv[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) yv[u] = (j0 + u < M) ? Wp[(size_t)(j0 + u) * K] : 0.0;
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int j = j0 + u;
-            if (j < M) {
-                const double a = t.am[j];
-                d = (t.bm0[j] + xl2 * t.cc[j]) + lam - a * cprev;
-                r = 1.0 / d;
-                cprev = t.cm[j] * r;
-                yprev = (yv[u] - a * yprev) * r;
-                Cp[(size_t)j * K] = cprev;
-                Wp[(size_t)j * K] = yprev;
-            }
-        }
-    }
-    double x = yprev;
-    for (int j0 = M - 2; j0 >= 0; j0 -= kU) {
-        double yv[kU], cv[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            yv[u] = (j0 - u >= 0) ? Wp[(size_t)(j0 - u) * K] : 0.0;
-            cv[u] = (j0 - u >= 0) ? Cp[(size_t)(j0 - u) * K] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u)
-            if (j0 - u >= 0) {
-                x = yv[u] - cv[u] * x;
-                Wp[(size_t)(j0 - u) * K] = x;
-            }
+    size_t o = (size_t)m * M * K + p;
+    double r = 1.0 / (t.bm0[0] + axis * t.ammin + xl2 * t.cc[0] + lam);
+    double c = t.cm[0] * r;
+    rec[o] = r;
+    mul[o] = c;
+    for (int j = 1; j < M; ++j) {
+        o += K;
+        r = 1.0 / ((t.bm0[j] + xl2 * t.cc[j]) + lam - t.am[j] * c);
+        c = t.cm[j] * r;
+        rec[o] = r;
+        mul[o] = c;
     }
 }
 
-// X_l(j,k) = sum_p V(k,p) W[l][j][p] for the interior (k < NZ, j < M).
-__global__ void __launch_bounds__(256) k_zinv_f64(DevTables t, Work w, int nb)
+// Radial sweeps (T_r(m) + lam_p) w = W_p with the plan's table, one thread per
+// (l, p), 128 / K modes per CTA: elimination down W, then back substitution,
+// both in place.  The table takes the division (and the multiplier's store and
+// reload) out of the recurrence, whose chain is then two dependent operations
+// a row.  A lone warp is bound by its instruction count and its loads' latency,
+// so the sweeps run over whole eight-row chunks, loaded one chunk ahead into a
+// second register set at constant offsets (KC = KMAX; 0: KMAX known at run time
+// only); AM is staged in shared memory (the streaming loads evict it from L1).
+// At 8 solves of 256x128x256: 0.53 ms with the divisions, 0.345 ms now, about
+// the time of its 330 MB per solve; with an eight-byte cp.async ring three
+// chunks deep instead of the registers 0.54 ms (bound by the copies' issue).
+template <int KC>
+__global__ void __launch_bounds__(128) k_thomas_f64(DevTables t, Work w)
 {
-    extern __shared__ double smem[];
-    double *Vs = smem;                  // [p][k], kPB x kPB
-    double *Ws = smem + kPB * kPB;      // [p][j], kPB x (kJT+1)
-    constexpr int ldw = kJT + 1;
-    const int NZ = t.NZ, tid = threadIdx.x;
-    for (int i = tid; i < kPB * kPB; i += blockDim.x) {
-        const int p = i / kPB, k = i % kPB;
-        Vs[i] = (k < NZ && p < NZ) ? t.V[(size_t)k * NZ + p] : 0.0;
+    constexpr int U = 8;
+    const int M = t.M, K = KC ? KC : t.K, p = threadIdx.x % K, b = blockIdx.y;
+    const int l = blockIdx.x * (blockDim.x / K) + threadIdx.x / K;
+    extern __shared__ double am[];
+    for (int j = threadIdx.x; j < M; j += blockDim.x) am[j] = t.am[j];
+    __syncthreads();
+    if (p >= t.NZ || l >= t.L) return;
+    double *Wp = w.W + (size_t)b * w.sW + (size_t)l * t.J * K + p;
+    const size_t tab = (size_t)mode_m(l, t.N) * M * K + p;
+    const double *rec = t.th_rec + tab, *mul = t.th_mul + tab;
+    double ya[U], ta[U], yb[U], tb[U];
+    const double *lw = Wp, *lt = rec;   // next rows to load
+    double prev = 0.0;
+    int j = 0;
+    auto load_down = [&](double (&y)[U], double (&r)[U]) {
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            y[i] = lw[i * K];
+            r[i] = __ldg(lt + i * K);
+        }
+        lw += U * K;
+        lt += U * K;
+    };
+    auto down = [&](const double (&y)[U], const double (&r)[U]) {
+        double *o = Wp + (size_t)j * K;
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            prev = (y[i] - am[j + i] * prev) * r[i];
+            o[i * K] = prev;
+        }
+        j += U;
+    };
+    int nf = M / U;
+    if (nf > 0) load_down(ya, ta);
+    for (int c = 0; c < nf; c += 2) {
+        if (c + 1 < nf) load_down(yb, tb);
+        down(ya, ta);
+        if (c + 2 < nf) load_down(ya, ta);
+        if (c + 1 < nf) down(yb, tb);
     }
-    const int njt = (t.M + kJT - 1) / kJT;
-    const long long items = (long long)nb * t.L * njt;
-    const int tk = tid / 8, tj = tid % 8, k0 = tk * 4, jj0 = tj * 4;
-    for (long long it = blockIdx.x; it < items; it += gridDim.x) {
-        const int jt = (int)(it % njt), l = (int)((it / njt) % t.L), b = (int)(it / ((long long)njt * t.L));
-        const int j0 = jt * kJT;
-        const double *Wl = w.W + (size_t)b * w.sW + (size_t)l * t.J * t.K;
-        __syncthreads();
-        for (int i = tid; i < kJT * NZ; i += blockDim.x) {
-            const int jj = i / NZ, p = i % NZ, j = j0 + jj;
-            Ws[p * ldw + jj] = (j < t.M) ? Wl[(size_t)j * t.K + p] : 0.0;
+    for (; j < M; ++j) {
+        prev = (Wp[(size_t)j * K] - am[j] * prev) * __ldg(rec + (size_t)j * K);
+        Wp[(size_t)j * K] = prev;
+    }
+    // rows M-2 .. 0, the odd ones first
+    double x = prev;
+    j = M - 2;
+    for (int n = (M - 1) % U; n > 0; --n, --j) {
+        x = Wp[(size_t)j * K] - __ldg(mul + (size_t)j * K) * x;
+        Wp[(size_t)j * K] = x;
+    }
+    lw = Wp + (ptrdiff_t)j * K;
+    lt = mul + (ptrdiff_t)j * K;
+    auto load_up = [&](double (&y)[U], double (&c)[U]) {
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            y[i] = lw[-i * K];
+            c[i] = __ldg(lt - i * K);
         }
-        __syncthreads();
-        double acc[4][4] = {};
-        for (int p = 0; p < NZ; ++p) {
-            double v[4], x[4];
+        lw -= U * K;
+        lt -= U * K;
+    };
+    auto up = [&](const double (&y)[U], const double (&c)[U]) {
+        double *o = Wp + (ptrdiff_t)j * K;
 #pragma unroll
-            for (int a = 0; a < 4; ++a) { v[a] = Vs[p * kPB + k0 + a]; x[a] = Ws[p * ldw + jj0 + a]; }
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[a][c] = fma(v[a], x[c], acc[a][c]);
+        for (int i = 0; i < U; ++i) {
+            x = y[i] - c[i] * x;
+            o[-i * K] = x;
         }
-        double *Xl = w.X + (size_t)b * w.sX + (size_t)l * t.K * t.J;
+        j -= U;
+    };
+    nf = (M - 1) / U;
+    if (nf > 0) load_up(ya, ta);
+    for (int c = 0; c < nf; c += 2) {
+        if (c + 1 < nf) load_up(yb, tb);
+        up(ya, ta);
+        if (c + 2 < nf) load_up(ya, ta);
+        if (c + 1 < nf) up(yb, tb);
+    }
+}
+
+// X_l(j,k) = sum_p V(k,p) W[l][j][p] for the interior (k < NZ, j < M).  A tile
+// of W is one contiguous run of rows.
+template <int KP, int MT>
+__global__ void __launch_bounds__(kZThreads, 1) k_zinv_f64(DevTables t, Work w, int nb)
+{
+    using Z = ZTile<KP, MT>;
+    extern __shared__ __align__(16) double smem[];   // [3][JT][LDW]
+    const int NZ = t.NZ, M = t.M, J = t.J, K = t.K, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wk = warp % Z::NWP, wj = warp / Z::NWP;
+    const int k = wk * 8 + lane / 4;
+    double va[Z::KS];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int k = k0 + a;
-            if (k < NZ)
+    for (int s = 0; s < Z::KS; ++s) {
+        const int p = 4 * s + lane % 4;
+        va[s] = (k < NZ && p < NZ) ? t.V[(size_t)k * NZ + p] : 0.0;
+    }
+    // columns p >= K of narrow grids and rows no copy reaches start as zeros
+    for (int i = tid; i < 3 * Z::kInvBuf; i += kZThreads) smem[i] = 0.0;
+    __syncthreads();
+    const int njt = (M + Z::JT - 1) / Z::JT;
+    const int items = nb * t.L * njt;
+    const int h = K / 2, hs = __ffs(h) - 1;   // KMAX is a power of two
+    auto load = [&](int it, double *T) {
+        if (it < items) {
+            const int q = it / njt, j0 = (it - q * njt) * Z::JT, rows = M - j0 < Z::JT ? M - j0 : Z::JT;
+            const double *Wl = w.W + ((size_t)q * J + j0) * K;
+            for (int i = tid; i < rows * h; i += kZThreads) {
+                const int r = i >> hs, c = 2 * (i & (h - 1));
+                z_cp16(T + r * Z::LDW + c, Wl + (size_t)r * K + c);
+            }
+        }
+        z_commit();
+    };
+    int it = blockIdx.x;
+    load(it, smem);
+    load(it + (int)gridDim.x, smem + Z::kInvBuf);
+    const bool pairs = (J & 1) == 0;
+    for (int buf = 0; it < items; it += gridDim.x, buf = buf == 2 ? 0 : buf + 1) {
+        z_wait<1>();
+        __syncthreads();
+        load(it + 2 * (int)gridDim.x, smem + (buf == 0 ? 2 : buf - 1) * Z::kInvBuf);
+        const double *T = smem + buf * Z::kInvBuf + (wj * 8 * MT + lane / 4) * Z::LDW + lane % 4;
+        double acc[MT][2] = {};
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int j = j0 + jj0 + c;
-                    if (j < t.M) Xl[(size_t)k * t.J + j] = acc[a][c];
-                }
+        for (int s = 0; s < Z::KS; ++s) {
+            double x[MT];
+#pragma unroll
+            for (int n = 0; n < MT; ++n) x[n] = T[8 * n * Z::LDW + 4 * s];
+#pragma unroll
+            for (int n = 0; n < MT; ++n) dmma(acc[n], va[s], x[n]);
+        }
+        const int q = it / njt, jt = it - q * njt;
+        double *Xl = w.X + (size_t)q * K * J;
+#pragma unroll
+        for (int n = 0; n < MT; ++n) {
+            const int j = jt * Z::JT + wj * 8 * MT + 8 * n + 2 * (lane % 4);
+            double *o = Xl + (size_t)k * J + j;
+            if (k < NZ && j + 1 < M && pairs) {
+                *reinterpret_cast<double2 *>(o) = make_double2(acc[n][0], acc[n][1]);
+            } else if (k < NZ) {
+                if (j < M) o[0] = acc[n][0];
+                if (j + 1 < M) o[1] = acc[n][1];
+            }
         }
     }
+}
+
+size_t thomas_table_doubles(int J, int K, int L) { return (size_t)(L / 2 + 1) * (J - 1) * K; }
+
+cudaError_t launch_thomas_table(const DevTables &t, double *rec, double *mul, cudaStream_t s)
+{
+    k_thomas_table<<<t.N + 1, 128, 0, s>>>(t, rec, mul);
+    return cudaGetLastError();
+}
+
+template <int KP, int MT>
+static cudaError_t solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s)
+{
+    using Z = ZTile<KP, MT>;
+    const int items = nb * t.L * ((t.M + Z::JT - 1) / Z::JT);   // at most 64 x 1024 x 512
+    // narrower tiles while the items do not fill the SMs twice
+    if constexpr (MT > 1)
+        if (items < 2 * num_sms) return solve_fp64<KP, MT / 2>(t, w, nb, num_sms, s);
+    cudaError_t e = ensure_smem((const void *)k_zfwd_f64<KP, MT>, Z::kFwdBytes);
+    if (e == cudaSuccess) e = ensure_smem((const void *)k_zinv_f64<KP, MT>, Z::kInvBytes);
+    auto sweep = KP == 16 && t.K < 16 ? k_thomas_f64<0> : k_thomas_f64<KP>;
+    if (e == cudaSuccess) e = ensure_smem((const void *)sweep, (size_t)t.M * sizeof(double));
+    if (e != cudaSuccess) return e;
+    const int grid = items < num_sms ? items : num_sms;
+    k_zfwd_f64<KP, MT><<<grid, kZThreads, Z::kFwdBytes, s>>>(t, w, nb);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    const int mpb = 128 / t.K;   // modes per CTA
+    sweep<<<dim3((t.L + mpb - 1) / mpb, nb), 128, (size_t)t.M * sizeof(double), s>>>(t, w);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    k_zinv_f64<KP, MT><<<grid, kZThreads, Z::kInvBytes, s>>>(t, w, nb);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s)
 {
-    const size_t sm1 = (size_t)(kPB * kPB + kPB * kJT) * sizeof(double);
-    const size_t sm3 = (size_t)(kPB * kPB + kPB * (kJT + 1)) * sizeof(double);
-    cudaError_t e = ensure_smem((const void *)k_zfwd_f64, sm1);
-    if (e == cudaSuccess) e = ensure_smem((const void *)k_zinv_f64, sm3);
-    if (e != cudaSuccess) return e;
-    if (t.NZ > kPB) return cudaErrorInvalidValue;
-    const int njt = (t.M + kJT - 1) / kJT;
-    const long long items = (long long)nb * t.L * njt;
-    const int grid = (int)(items < num_sms ? items : num_sms);
-    k_zfwd_f64<<<grid, 256, sm1, s>>>(t, w, nb);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_thomas_f64<<<dim3(t.L, 1, nb), 128, 0, s>>>(t, w);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_zinv_f64<<<grid, 256, sm3, s>>>(t, w, nb);
-    return cudaGetLastError();
+    if (t.K <= 16) return solve_fp64<16, 4>(t, w, nb, num_sms, s);
+    if (t.K <= 32) return solve_fp64<32, 8>(t, w, nb, num_sms, s);
+    if (t.K <= 64) return solve_fp64<64, 8>(t, w, nb, num_sms, s);
+    if (t.K <= 128) return solve_fp64<128, 8>(t, w, nb, num_sms, s);
+    return cudaErrorInvalidValue;
 }
-
 
 }  // namespace chy
