@@ -8,6 +8,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "chy_pot3.h"
@@ -90,6 +91,33 @@ static int check_device(const chy_plan *p)
     return CHY_OK;
 }
 
+// The BLKTRI-order path's pivot table.  It only saves time, so it is left out
+// where it would take more than kBlkTableMax bytes or leave less than half of
+// the device's memory free, or where a pivot is out of the range its quotients
+// need.
+static constexpr size_t kBlkTableMax = (size_t)2 << 30;
+static int make_blk_table(chy_plan *p, int nroots)
+{
+    const size_t n = blk_table_doubles(p->t.M, p->t.L, nroots), bytes = n * sizeof(double) + 256;
+    size_t free_b = 0, total = 0;
+    if (n == 0 || bytes > kBlkTableMax) return CHY_OK;
+    CHY_CUDA(cudaMemGetInfo(&free_b, &total));
+    if (free_b < bytes + total / 2) return CHY_OK;
+    if (cudaMalloc(&p->d_blktab, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        p->d_blktab = nullptr;
+        return CHY_OK;
+    }
+    int *bad = (int *)(p->d_blktab + n), h_bad = 0;
+    CHY_CUDA(cudaMemset(bad, 0, sizeof(int)));
+    CHY_CUDA(launch_blk_table(p->t, nroots, p->d_blktab, bad, cudaStreamLegacy));
+    CHY_CUDA(cudaMemcpy(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost));
+    p->blktab_bytes = bytes;
+    p->t.blk.tab = p->d_blktab;
+    if (h_bad) chy_internal_drop_blk_table(p);
+    return CHY_OK;
+}
+
 extern "C" {
 
 void chy_grid_defaults(chy_grid *g, int jmax, int kmax, int lmax)
@@ -141,6 +169,7 @@ void chy_plan_destroy(chy_plan *p)
             if (e) cudaEventDestroy(e);
     cudaFree(p->d_tables);
     cudaFree(p->d_work);
+    cudaFree(p->d_blktab);
     cudaFree(p->stage);
     cudaFree(p->coef_dev);
     for (int i = 0; i < chy_plan::kStageSlots; i++) {
@@ -211,8 +240,19 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     size_t o_am = pk.vec(hp.am), o_cmv = pk.vec(hp.cm), o_cc = pk.vec(hp.cc), o_bm0 = pk.vec(hp.bm0), o_xl = pk.vec(hp.xlamm);
     size_t o_an = pk.vec(hp.an), o_bn = pk.vec(hp.bn), o_cn = pk.vec(hp.cn);
     size_t o_U = pk.vec(hp.U), o_V = pk.vec(hp.V), o_lam = pk.vec(hp.lam);
+    std::vector<double> roots;   // distinct shifts of the schedule
+    bool blk_none = false;
+    size_t o_brt = 0;
     size_t o_bst = 0, o_bpg = 0, o_btk = 0, o_bsg = 0, o_bmt = 0;
     if (precision == CHY_PREC_FP64_BLKTRI) {
+        std::unordered_map<double, int> index;
+        for (BlkStep &st : bs.steps) {
+            const auto at = index.emplace(st.rt, (int)roots.size());
+            if (at.second) roots.push_back(st.rt);
+            st.pad = at.first->second;
+            blk_none |= st.post == BLK_NONE;
+        }
+        o_brt = pk.vec(roots);
         o_bst = pk.vec(bs.steps);
         o_bpg = pk.vec(bs.progs);
         o_btk = pk.vec(bs.tasks);
@@ -287,6 +327,8 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
         t.blk.tasks = (const BlkTask *)(D + o_btk);
         t.blk.stages = (const BlkStage *)(D + o_bsg);
         t.blk.bmt = (const double *)(D + o_bmt);
+        t.blk.roots = (const double *)(D + o_brt);
+        t.blk.ntab = blk_table_blocks(hp.L);
     }
     chy_mixed_bind_tables(p, D + o_ext);
 
@@ -330,6 +372,13 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     chy_mixed_bind_work(p, q);
     CHY_CUDA(cudaMemset(p->d_work, 0, p->work_bytes));
     p->nvol = (size_t)(hp.J + 2) * (hp.K + 2) * hp.L;
+    if (blk && !blk_none) {
+        st = make_blk_table(p, (int)roots.size());
+        if (st != CHY_OK) {
+            chy_plan_destroy(p);
+            return st;
+        }
+    }
     CHY_CUDA(cudaMallocHost(&p->h_diag, sizeof(double) * kDiagPart * max_batch));
     *out = p;
     return CHY_OK;
@@ -509,7 +558,7 @@ int chy_source_binary(chy_plan *p, const chy_source_args *a, const chy_binary *b
 long long chy_plan_device_bytes(const chy_plan *p)
 {
     if (!p) return 0;
-    return (long long)(p->table_bytes + p->work_bytes + p->stage_bytes + p->coef_bytes + chy_mixed_iterate_bytes(p));
+    return (long long)(p->table_bytes + p->blktab_bytes + p->work_bytes + p->stage_bytes + p->coef_bytes + chy_mixed_iterate_bytes(p));
 }
 
 long long chy_plan_bytes_per_solve(const chy_plan *p)
@@ -1001,6 +1050,16 @@ extern "C" int chy_autotune_multi(int n, chy_plan *const *plans, const double *c
         out->candidates = tried;
     }
     return CHY_OK;
+}
+
+size_t chy_internal_drop_blk_table(chy_plan *p)
+{
+    const size_t bytes = p->blktab_bytes;
+    cudaFree(p->d_blktab);   // waits for the launches that read it
+    p->d_blktab = nullptr;
+    p->blktab_bytes = 0;
+    p->t.blk.tab = nullptr;
+    return bytes;
 }
 
 int chy_internal_run_batch(chy_plan *p, const BatchPtrs &bp, int nb, cudaStream_t s) { return run_batch(p, bp, nb, s); }

@@ -39,7 +39,7 @@ struct BlkStep {
     double rt;     // shift BD(ID) of the pass
     double coef;   // c of Y = Y + c W (RT - BM1/BM2 root) or Y = c W (AA(IA))
     int post;      // BLK_*
-    int pad;
+    int pad;       // device copy: index of rt among the distinct shifts
 };
 
 struct BlkProg {       // one PRDCT call

@@ -57,6 +57,11 @@ struct BlkDev {
     const BlkTask *tasks;
     const BlkStage *stages;
     const double *bmt;
+    // pivots of every distinct shift (BlkStep::pad indexes it), or null:
+    // [root][ntab mode blocks][z, l, D][M][32] (k_blktri.cu); block b <= LMAX/64 holds
+    // the modes 32 b + lane, the later ones' m repeats block b - LMAX/64's
+    const double *tab, *roots;
+    int ntab;
 };
 
 struct DevTables {
@@ -158,6 +163,11 @@ cudaError_t launch_thomas_table(const DevTables &t, double *rec, double *mul, cu
 cudaError_t launch_solve_blk(const DevTables &t, const Work &w, int nb, int num_sms, int nw, int ctas_per_sm,
                              cudaStream_t s, int *launches);
 bool blk_schedule_valid(int nw, int ctas_per_sm);
+// The pivot table of the BLKTRI-order path: its size (0: this M runs without
+// one), its mode blocks and its kernel.
+size_t blk_table_doubles(int M, int L, int nroots);
+int blk_table_blocks(int L);
+cudaError_t launch_blk_table(const DevTables &t, int nroots, double *tab, int *bad, cudaStream_t s);
 // Its work-space sizes in doubles: BVEC for nb solves, BSCR for a plan of max_batch.
 size_t blk_vector_doubles(const DevTables &t, int nb);
 size_t blk_scratch_doubles(const DevTables &t, int max_batch, int num_sms);

@@ -31,6 +31,8 @@ struct chy_plan {
     int streams = 0;               // chy_solve_multi: grids in flight at once (default 8)
     char *d_tables = nullptr;
     size_t table_bytes = 0;
+    double *d_blktab = nullptr;    // BLKTRI order: pivot table (null: passes divide)
+    size_t blktab_bytes = 0;
     char *d_work = nullptr;
     size_t work_bytes = 0;
     chy::Work w{};
@@ -119,6 +121,10 @@ int chy_internal_fail(int code, const char *msg);
 
 // One launch sequence over nb device-pointer solves (api.cu).
 int chy_internal_run_batch(chy_plan *p, const chy::BatchPtrs &bp, int nb, cudaStream_t s);
+
+// Gives back a plan's BLKTRI pivot table (its passes divide from then on) once
+// the device has finished with it; returns the bytes freed (api.cu).
+size_t chy_internal_drop_blk_table(chy_plan *p);
 
 // Mixed-precision mode solve (k_mixed.cu).
 bool chy_mixed_supported(const chy::HostPlan *hp);

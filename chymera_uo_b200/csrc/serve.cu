@@ -249,6 +249,14 @@ int chy_server::make_class(Request *rq, SizeClass **out)
         }
     }
     c->last_use = Clock::now();
+    // over budget: first the BLKTRI pivot tables go, which only save time (this
+    // thread is the only one that launches with these plans)
+    auto drop_tables = [&](SizeClass &o) {
+        for (Lane &ln : o.lanes)
+            if (plan_bytes > budget - arena.size) plan_bytes -= chy_internal_drop_blk_table(ln.plan);
+    };
+    drop_tables(*c);
+    for (auto &kv : classes) drop_tables(*kv.second);
     // plans count against the budget left after the arena: drop idle classes
     // (least recently used first) to make room, else give up on this grid
     while (plan_bytes > budget - arena.size) {
