@@ -239,6 +239,7 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     size_t o_bin = pk.vec(hp.jk_bin), o_hout = pk.vec(hp.jk_hout);
     size_t o_am = pk.vec(hp.am), o_cmv = pk.vec(hp.cm), o_cc = pk.vec(hp.cc), o_bm0 = pk.vec(hp.bm0), o_xl = pk.vec(hp.xlamm);
     size_t o_an = pk.vec(hp.an), o_bn = pk.vec(hp.bn), o_cn = pk.vec(hp.cn);
+    const size_t o_zw = pk.vec(hp.zw), o_tc = pk.vec(hp.term_col);
     size_t o_U = pk.vec(hp.U), o_V = pk.vec(hp.V), o_lam = pk.vec(hp.lam);
     std::vector<double> roots;   // distinct shifts of the schedule
     bool blk_none = false;
@@ -306,7 +307,8 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     t.bm0 = (const double *)(D + o_bm0); t.xlamm = (const double *)(D + o_xl);
     t.an = (const double *)(D + o_an); t.bn = (const double *)(D + o_bn); t.cn = (const double *)(D + o_cn);
     t.U = (const double *)(D + o_U); t.V = (const double *)(D + o_V); t.lam = (const double *)(D + o_lam);
-    for (int i = 0; i < 11; i++) t.zx[i] = hp.zx[i];
+    t.zw = (const double *)(D + o_zw);
+    t.term_col = (const int *)(D + o_tc);
     if (nth) {
         double *rec = (double *)(D + o_dev), *mul = rec + nth;
         t.th_rec = rec;

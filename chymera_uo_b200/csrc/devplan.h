@@ -88,7 +88,8 @@ struct DevTables {
     const double *U, *V, *lam;
     // radial elimination table of the FP64 path, [N+1][M][K]: pivot reciprocals, multipliers
     const double *th_rec, *th_mul;
-    double zx[11];
+    const double *zw;               // ZAXPHI's step weights (HostPlan::zw)
+    const int *term_col;            // [132] column of (part, term), or -1
     BlkDev blk;                     // CHY_PREC_FP64_BLKTRI plans only
 };
 

@@ -24,6 +24,10 @@ namespace chy {
 // ring-table slice of a sub-chunk is loaded once and serves up to kSubBatch
 // solves, two solves per pass.  Every column sum keeps its order, whatever
 // the pairing.
+// Latency-bound when few solves share the launch: the table slice arrives by
+// asynchronous copies while a thread's moments are in flight together (one solve
+// of 256x128x256 28 -> 16.4 us, of 64x32x64 14.5 -> 6.6 us, 32 solves 236 -> 225
+// us against loads one after another behind the slice).
 constexpr int kSubBatch = 8;
 constexpr int kSubThreads = 512;
 __global__ void __launch_bounds__(kSubThreads) k_bdy_sub(DevTables t, Work w, int nb, int spp)
@@ -32,23 +36,55 @@ __global__ void __launch_bounds__(kSubThreads) k_bdy_sub(DevTables t, Work w, in
     const int RL = t.srow, NT_ = t.ntrm;
     double *s_row = smem;                                      // [ns][RL]: TERM, r^-(2l+1), DV
     double *s_mom = smem + kSubChunk * RL;                     // [spp][ns][21]
-    int *s_ring = reinterpret_cast<int *>(s_mom + (size_t)spp * kSubChunk * 21);   // [ns] ring index
     const int sc = blockIdx.x;
     const int s0 = t.sub_start[sc], s1 = t.sub_start[sc + 1], ns = s1 - s0;
 
     // per ring, geometry from the plan (TERM(I) of pot/boundary.f:385-502,
-    // r^-(2l+1) of :587, DV of :516)
-    for (int i = threadIdx.x; i < ns * RL; i += blockDim.x) s_row[i] = t.sterm[(size_t)s0 * RL + i];
-    for (int i = threadIdx.x; i < ns; i += blockDim.x) s_ring[i] = t.ring_sorted[s0 + i];
+    // r^-(2l+1) of :587, DV of :516): asynchronous copies, under way while the
+    // moments are gathered into registers
+    const double *row = t.sterm + (size_t)s0 * RL;
+    if ((RL & 1) == 0) {
+        for (int i = threadIdx.x; i < ns * RL / 2; i += blockDim.x)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(s_row + 2 * i)),
+                         "l"(row + 2 * i)
+                         : "memory");
+    } else {
+        for (int i = threadIdx.x; i < ns * RL; i += blockDim.x)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(s_row + i)),
+                         "l"(row + i)
+                         : "memory");
+    }
     const int b0 = blockIdx.z * kSubBatch, b1 = min(nb, b0 + kSubBatch);
     for (int b = b0; b < b1; b += spp) {
         const int nsl = min(spp, b1 - b);
-        __syncthreads();   // s_row loaded / s_mom of the previous solves consumed
-        // DV * moments of these solves
-        for (int it = threadIdx.x; it < nsl * ns * 21; it += blockDim.x) {
-            const int sl = it / (ns * 21), rq = it % (ns * 21), r = rq / 21, q = rq % 21;
-            const double *mom = w.mom + (size_t)(b + sl) * w.smom;
-            s_mom[((size_t)sl * kSubChunk + r) * 21 + q] = s_row[r * RL + NT_ + 11] * mom[(size_t)q * t.nring + s_ring[r]];
+        // the moments of these solves, kGather of a thread's in flight at once;
+        // consecutive threads take consecutive rings of one moment
+        constexpr int kGather = 10;
+        const int total = nsl * 21 * kSubChunk;   // rings ns .. 63 of each moment are skipped
+        for (int g0 = 0; g0 < total; g0 += kGather * blockDim.x) {
+            double v[kGather];
+#pragma unroll
+            for (int u = 0; u < kGather; ++u) {
+                const int it = g0 + u * blockDim.x + threadIdx.x;
+                const int r = it % kSubChunk, sl = it / (21 * kSubChunk), q = it / kSubChunk - 21 * sl;
+                v[u] = 0.0;
+                if (it < total && r < ns) {
+                    v[u] = w.mom[(size_t)(b + sl) * w.smom + (size_t)q * t.nring + __ldg(t.ring_sorted + s0 + r)];
+                }
+            }
+            if (g0 == 0) {
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncthreads();   // s_row landed / s_mom of the previous solves consumed
+            }
+            // DV * moments
+#pragma unroll
+            for (int u = 0; u < kGather; ++u) {
+                const int it = g0 + u * blockDim.x + threadIdx.x;
+                const int r = it % kSubChunk, sl = it / (21 * kSubChunk), q = it / kSubChunk - 21 * sl;
+                if (it < total && r < ns) {
+                    s_mom[((size_t)sl * kSubChunk + r) * 21 + q] = s_row[r * RL + NT_ + 11] * v[u];
+                }
+            }
         }
         __syncthreads();
         // Column col's inside and outside sums of these solves, each as four
@@ -109,22 +145,23 @@ __global__ void __launch_bounds__(kSubThreads) k_bdy_sub(DevTables t, Work w, in
     }
 }
 
-// Grid: (ceil(2*ncol / 32), 1, batch), 512 threads: lane i of every warp
-// takes column 32 blockIdx.x + i of the [2][ncol] row (inside sums, then
-// outside sums), so each row is read and written in one coalesced piece;
-// warp s takes the s-th of kScanRuns consecutive runs of sub-chunks in scan
-// order.
+// Grid: (ceil(2*ncol / kScanCols), 1, batch): half a warp takes kScanCols
+// consecutive columns of the [2][ncol] row (inside sums, then outside sums), so
+// each row is read and written in one 128-byte piece, and half-warp s the s-th of
+// kScanRuns consecutive runs of sub-chunks in scan order.  Latency-bound: with
+// 16 runs, each read twice eight loads at a time, one solve of 256x128x256 (872
+// sub-chunks) took 17.2 us, now 7.8 us.
 // scan[i][0][col] = sum of inside sums of sub-chunks < i (prefix from the
 // innermost ring); scan[i][1][col] = sum of outside sums of sub-chunks >= i
 // (suffix from the outermost ring).  Each run is summed in order, the run
 // totals are added in order, and every prefix is that base plus the run's
 // running sum: a fixed order, so the result is bit-reproducible.
-constexpr int kScanRuns = 16;
-__global__ void __launch_bounds__(32 * kScanRuns) k_bdy_scan(DevTables t, Work w)
+constexpr int kScanCols = 16, kScanRuns = 64, kScanRegs = 16;
+__global__ void __launch_bounds__(kScanCols *kScanRuns) k_bdy_scan(DevTables t, Work w)
 {
-    __shared__ double run_tot[kScanRuns][32];
-    const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5, b = blockIdx.z;
-    const int cc = blockIdx.x * 32 + lane, ld = 2 * t.ncol;
+    __shared__ double run_tot[kScanRuns][kScanCols];
+    const int lane = threadIdx.x % kScanCols, seg = threadIdx.x / kScanCols, b = blockIdx.z;
+    const int cc = blockIdx.x * kScanCols + lane, ld = 2 * t.ncol;
     const bool live = cc < ld, out = cc >= t.ncol;
     const double *__restrict__ sub = w.sub + (size_t)b * w.ssub;
     double *__restrict__ scan = w.scan + (size_t)b * w.sscan;
@@ -132,40 +169,57 @@ __global__ void __launch_bounds__(32 * kScanRuns) k_bdy_scan(DevTables t, Work w
     const int lo = min(seg * per, ns), hi = min(lo + per, ns);
     // position p in scan order -> sub-chunk index
     auto idx = [&](int p) { return out ? ns - 1 - p : p; };
-    // loads go eight at a time, so that their latencies overlap; the sums
-    // stay in order
+    // a run's loads go kU at a time, so that their latencies overlap; runs of
+    // up to kScanRegs sub-chunks stay in registers for the second pass.  The
+    // sums stay in order.
     constexpr int kU = 8;
+    const bool held = per <= kScanRegs;
+    double v[kScanRegs];
     double local = 0.0;
-    if (live)
-        for (int p0 = lo; p0 < hi; p0 += kU) {
-            double v[kU];
+    if (live) {
+        if (held) {
 #pragma unroll
-            for (int u = 0; u < kU; ++u) v[u] = p0 + u < hi ? sub[(size_t)idx(p0 + u) * ld + cc] : 0.0;
+            for (int u = 0; u < kScanRegs; ++u) v[u] = lo + u < hi ? sub[(size_t)idx(lo + u) * ld + cc] : 0.0;
 #pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (p0 + u < hi) local = local + v[u];
+            for (int u = 0; u < kScanRegs; ++u)
+                if (lo + u < hi) local = local + v[u];
+        } else {
+            for (int p0 = lo; p0 < hi; p0 += kU) {
+#pragma unroll
+                for (int u = 0; u < kU; ++u) v[u] = p0 + u < hi ? sub[(size_t)idx(p0 + u) * ld + cc] : 0.0;
+#pragma unroll
+                for (int u = 0; u < kU; ++u)
+                    if (p0 + u < hi) local = local + v[u];
+            }
         }
+    }
     run_tot[seg][lane] = local;
     __syncthreads();
     double base = 0.0;
     for (int i = 0; i < seg; ++i) base = base + run_tot[i][lane];
     if (!live) return;
     double run = base;
-    for (int p0 = lo; p0 < hi; p0 += kU) {
-        double v[kU];
+    auto put = [&](int p, double x) {
+        const size_t at = (size_t)idx(p) * ld + cc;
+        if (!out) {
+            scan[at] = run;
+            run = run + x;
+        } else {
+            run = run + x;
+            scan[at] = run;
+        }
+    };
+    if (held) {
 #pragma unroll
-        for (int u = 0; u < kU; ++u) v[u] = p0 + u < hi ? sub[(size_t)idx(p0 + u) * ld + cc] : 0.0;
+        for (int u = 0; u < kScanRegs; ++u)
+            if (lo + u < hi) put(lo + u, v[u]);
+    } else {
+        for (int p0 = lo; p0 < hi; p0 += kU) {
 #pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            if (p0 + u >= hi) break;
-            const size_t at = (size_t)idx(p0 + u) * ld + cc;
-            if (!out) {
-                scan[at] = run;
-                run = run + v[u];
-            } else {
-                run = run + v[u];
-                scan[at] = run;
-            }
+            for (int u = 0; u < kU; ++u) v[u] = p0 + u < hi ? sub[(size_t)idx(p0 + u) * ld + cc] : 0.0;
+#pragma unroll
+            for (int u = 0; u < kU; ++u)
+                if (p0 + u < hi) put(p0 + u, v[u]);
         }
     }
     if (seg == kScanRuns - 1) scan[(size_t)ns * ld + cc] = out ? 0.0 : run;   // the inside total
@@ -178,13 +232,13 @@ cudaError_t launch_bdy_sums(const DevTables &t, const Work &w, int nb, cudaStrea
     if (4 * t.ncol > kSubThreads) return cudaErrorInvalidConfiguration;
     const int spp = nb >= 2 ? 2 : 1;
     const int threads = ((4 * t.ncol + 31) / 32) * 32;
-    const size_t sm = (size_t)kSubChunk * (t.srow + 21 * spp) * sizeof(double) + (size_t)kSubChunk * sizeof(int);
+    const size_t sm = (size_t)kSubChunk * (t.srow + 21 * spp) * sizeof(double);
     cudaError_t e = ensure_smem((const void *)k_bdy_sub, sm);
     if (e != cudaSuccess) return e;
     k_bdy_sub<<<dim3(t.nsub, 1, (nb + kSubBatch - 1) / kSubBatch), threads, sm, s>>>(t, w, nb, spp);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_bdy_scan<<<dim3((2 * t.ncol + 31) / 32, 1, nb), 32 * kScanRuns, 0, s>>>(t, w);
+    k_bdy_scan<<<dim3((2 * t.ncol + kScanCols - 1) / kScanCols, 1, nb), kScanCols * kScanRuns, 0, s>>>(t, w);
     return cudaGetLastError();
 }
 

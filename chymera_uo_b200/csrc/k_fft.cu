@@ -535,30 +535,45 @@ __global__ void __launch_bounds__(256) k_forward(DevTables t, BatchPtrs bp, Work
 // s_m = 2 sum_L TRMTOT(2,(L,m)).  POT3 then transforms the boundary columns
 // (pot/pot3.f:93-140); the transform being linear, the modes are the same
 // combination of the recorded transforms of {1, cos m psi, sin m psi}.
+// Latency-bound: every load of a thread is issued before the first is used (one
+// solve of 64x32x64 9.0 -> 5.8 us, 32 of 256x128x256 72 -> 68 us).
 __global__ void __launch_bounds__(256) k_bdy_synth(DevTables t, Work w)
 {
     constexpr int kPts = 8;
     __shared__ double trm[kPts][132];
     __shared__ double cq[kPts][21];
-    __shared__ int colidx[132];
     const int q0 = blockIdx.x * kPts, b = blockIdx.z, L = t.L;
     const double *scan = w.scan + (size_t)b * w.sscan;
-
-    for (int i = threadIdx.x; i < 132; i += blockDim.x) colidx[i] = -1;
-    __syncthreads();
-    for (int i = threadIdx.x; i < t.ncol; i += blockDim.x) colidx[t.col_part[i] * 66 + t.col_term[i]] = i;
-    __syncthreads();
-    for (int i = threadIdx.x; i < kPts * 132; i += blockDim.x) {
-        const int c = i / 132, r = i % 132, part = r / 66, term = r % 66, q = q0 + c;
-        double v = 0.0;
-        if (q < t.njk && term < t.ntrm) {
-            const int col = colidx[part * 66 + term];
-            const size_t srow = (size_t)t.jk_sub[q] * 2 * t.ncol;
-            const double min_ = col >= 0 ? scan[srow + col] : 0.0;
-            const double mout = col >= 0 ? scan[srow + t.ncol + col] : 0.0;
-            v = t.jk_bin[(size_t)q * 66 + term] * min_ + t.jk_hout[(size_t)q * 66 + term] * mout;
+    // one azimuth l per thread: its 21 basis values serve the block's kPts
+    // boundary points; the first azimuth's are on their way from the start
+    double f[21];
+    int l = threadIdx.x;
+    if (l < L) {
+#pragma unroll
+        for (int p = 0; p < 21; ++p) f[p] = __ldg(t.fbasis + (size_t)p * L + l);
+    }
+    // TRMTOT: all of a thread's loads in flight together
+    constexpr int NT = (kPts * 132 + 255) / 256;
+    double vi[NT], vo[NT], bi[NT], bo[NT];
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+        const int i = threadIdx.x + 256 * u, c = i / 132, r = i % 132, term = r % 66, q = q0 + c;
+        vi[u] = vo[u] = bi[u] = bo[u] = 0.0;
+        if (c < kPts && q < t.njk && term < t.ntrm) {
+            const int col = __ldg(t.term_col + r);
+            const size_t srow = (size_t)__ldg(t.jk_sub + q) * 2 * t.ncol;
+            if (col >= 0) {
+                vi[u] = scan[srow + col];
+                vo[u] = scan[srow + t.ncol + col];
+            }
+            bi[u] = __ldg(t.jk_bin + (size_t)q * 66 + term);
+            bo[u] = __ldg(t.jk_hout + (size_t)q * 66 + term);
         }
-        trm[c][r] = v;
+    }
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+        const int i = threadIdx.x + 256 * u, c = i / 132, r = i % 132;
+        if (c < kPts) trm[c][r] = bi[u] * vi[u] + bo[u] * vo[u];
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kPts * 21; i += blockDim.x) {
@@ -569,13 +584,8 @@ __global__ void __launch_bounds__(256) k_bdy_synth(DevTables t, Work w)
         cq[c][q] = -t.grav * (q == 0 ? s : 2.0 * s);
     }
     __syncthreads();
-    // one azimuth l per thread: its 21 basis values are read once and serve
-    // the block's kPts boundary points
     double *X = w.X + (size_t)b * w.sX;
-    for (int l = threadIdx.x; l < L; l += blockDim.x) {
-        double f[21];
-#pragma unroll
-        for (int p = 0; p < 21; ++p) f[p] = __ldg(t.fbasis + (size_t)p * L + l);
+    while (l < L) {
 #pragma unroll 2
         for (int c = 0; c < kPts; ++c) {
             const int q = q0 + c;
@@ -585,6 +595,11 @@ __global__ void __launch_bounds__(256) k_bdy_synth(DevTables t, Work w)
                 for (int p = 0; p < 21; ++p) v = __fma_rn(cq[c][p], f[p], v);
                 X[((size_t)l * t.K + t.jk_k[q]) * t.J + t.jk_j[q]] = v;
             }
+        }
+        l += blockDim.x;
+        if (l < L) {
+#pragma unroll
+            for (int p = 0; p < 21; ++p) f[p] = __ldg(t.fbasis + (size_t)p * L + l);
         }
     }
 }
@@ -630,33 +645,54 @@ __global__ void k_coef(DevTables t, Work w)
 // (pot/pot3.f:293-296).
 // ZAXPHI's Neville extrapolation to r = 0 (pot/pot3.f:354-378) for azimuth
 // l from NP samples PHI(2.., K, L) and PHI(2.., K, L+N) at the abscissae ZX,
-// every operation as the reference orders it.  The table P2 is held as its
-// live tail Q(S) = P2(II+S), which shifts down one place per step II, so
-// that every index is static and the table stays in registers.
-template <int NP, class F>
-__device__ __forceinline__ double neville_axis(const double (&zx)[11], F sample, int l, int lm)
+// every operation as the reference orders it.  Lane s of a group of G lanes
+// (8 up to NPOINT = 8, else 16) holds P2(II+S), the live tail of the table, which
+// shifts down one lane per step II: a step's quotients run side by side.
+// The weights depend on ZX only: XR = 0, so a step's numerator is
+// P1*XRATIO - P2 and its divisor XRATIO - 1.  zw (shared memory) holds per step
+// and place XRATIO, the divisor b, and 1/b as z + r (z the reciprocal rounded
+// towards zero, r the rest): the quotient a/b is q = RN(a z + RN(a r)), which
+// the last test shows to be a/b rounded to nearest (its remainder is below half
+// an ulp with room for the error of z + r).  Where a test fails in any lane of
+// the warp, or a dividend is zero, tiny or not finite, the warp runs its tables
+// again with divisions.  All 32 lanes of a warp call this.  At
+// LMAX = 64 it takes an axis tile 1.9k cycles; by one thread per azimuth with
+// divisions the tile set the kernel's time (11.7 us for one solve of 64x32x64,
+// now 7.8 us).
+template <class F>
+__device__ __forceinline__ double neville_axis(const double *zw, int np, int G, F sample, int l, int lm)
 {
-    constexpr int ichk = NP % 2, num = (NP - ichk) / 2, jsp = num + 1;
-    double q[NP];   // q[i] = P2(i + 1) before the first step
-#pragma unroll
-    for (int jj = 2; jj <= jsp; ++jj) {
-        q[num + (jj - 1) - 1] = sample(l, jj - 2);
-        q[num - (jj - 2) - 1] = sample(l + lm, jj - 2);
+    const int s = threadIdx.x & (G - 1), num = np / 2;
+    const double first = s < num ? sample(l + lm, num - 1 - s) : s < np ? sample(l, s - num) : 1.0;
+    double q = first;
+    bool ok = true;
+    auto weights = [&](int ii) {   // past the table: a quotient by one
+        const double2 *wt = reinterpret_cast<const double2 *>(zw) + 2 * (ii * (np - 1) + s);
+        double4 c = make_double4(0.0, 1.0, 1.0, 0.0);
+        if (s < np - 1) {
+            const double2 c0 = wt[0], c1 = wt[1];
+            c = make_double4(c0.x, c0.y, c1.x, c1.y);
+        }
+        return c;
+    };
+    for (int ii = 0; ii < np - 1; ++ii) {
+        const double4 c = weights(ii);
+        const double p1 = __shfl_sync(0xffffffffu, q, 0, G), p2 = __shfl_down_sync(0xffffffffu, q, 1, G);
+        const double a = p1 * c.x - p2;
+        const double pl = __dmul_rn(a, c.w), qt = __fma_rn(a, c.z, pl);
+        const double r = __dadd_rn(__fma_rn(a, c.z, -qt), pl);
+        ok = ok & (__fma_rn(r, 1.0 + 0x1p-40, qt) == qt) & (fabs(a) > 0x1p-800);
+        q = qt;
     }
-    if constexpr (ichk == 1) q[num + num] = sample(l, num);
-    const double xpoint = 0.0;
-#pragma unroll 1
-    for (int ii = 1; ii <= NP - 1; ++ii) {
-        const double p1 = q[0], xinv = 1.0 / zx[ii], xr = xpoint * xinv;
-#pragma unroll
-        for (int s = 0; s < NP - 1; ++s) {
-            if (s < NP - ii) {   // JJ = II + 1 + S
-                const double xratio = zx[ii + 1 + s] * xinv, pp = q[s + 1];
-                q[s] = (p1 * (xratio - xr) + pp * (xr - 1.0)) / (xratio - 1.0);
-            }
+    if (!__all_sync(0xffffffffu, ok)) {
+        q = first;
+        for (int ii = 0; ii < np - 1; ++ii) {
+            const double4 c = weights(ii);
+            const double p1 = __shfl_sync(0xffffffffu, q, 0, G), p2 = __shfl_down_sync(0xffffffffu, q, 1, G);
+            q = (p1 * c.x - p2) / c.y;
         }
     }
-    return q[0];
+    return __shfl_sync(0xffffffffu, q, 0, G);
 }
 
 // STARPHI of the cell (j, k, l) of PHI(J+2, K+2, L), 0-based, with the star at
@@ -723,6 +759,9 @@ __global__ void __launch_bounds__(256) k_inverse(DevTables t, BatchPtrs bp, Work
     const int j0 = blockIdx.x * T::TC, k = blockIdx.y, b = blockIdx.z;
     const double *X = w.X + (size_t)b * w.sX;
     double *phi = bp.phi[b];
+    double *zw = reinterpret_cast<double *>(tbar + 2);   // ZAXPHI's weights (axis tiles)
+    if (j0 == 0)
+        for (int i = threadIdx.x; i < 4 * (t.npoint - 1) * (t.npoint - 1); i += blockDim.x) zw[i] = __ldg(t.zw + i);
 
     // xmode 2: two sets of TMA boxes of the tensor map over X (J, K, L x batch),
     // TC columns x one K x up to 256 modes: modes 0..N-1 into rows 0..N-1 and
@@ -825,22 +864,16 @@ __global__ void __launch_bounds__(256) k_inverse(DevTables t, BatchPtrs bp, Work
         }
         // ZAXPHI: Neville extrapolation to r = 0 across +-RHF (pot/pot3.f:354-378)
         const int lm = L / 2;
-        for (int l = threadIdx.x; l < lm; l += blockDim.x) {
-            double ph;
-            switch (t.npoint) {   // 2..10, checked at plan creation
-            case 2: ph = neville_axis<2>(t.zx, sample, l, lm); break;
-            case 3: ph = neville_axis<3>(t.zx, sample, l, lm); break;
-            case 4: ph = neville_axis<4>(t.zx, sample, l, lm); break;
-            case 5: ph = neville_axis<5>(t.zx, sample, l, lm); break;
-            case 6: ph = neville_axis<6>(t.zx, sample, l, lm); break;
-            case 7: ph = neville_axis<7>(t.zx, sample, l, lm); break;
-            case 8: ph = neville_axis<8>(t.zx, sample, l, lm); break;
-            case 9: ph = neville_axis<9>(t.zx, sample, l, lm); break;
-            default: ph = neville_axis<10>(t.zx, sample, l, lm); break;
+        const int G = t.npoint <= 8 ? 8 : 16, s = threadIdx.x & (G - 1);
+        for (int l0 = 0; l0 < lm; l0 += blockDim.x / G) {
+            // groups past the last azimuth repeat it
+            const int l = min(l0 + (int)threadIdx.x / G, lm - 1);
+            const double ph = neville_axis(zw, t.npoint, G, sample, l, lm);
+            if (s == 0) red[l] = ph;
+            if (s < 2) {
+                const int lo = l + s * lm;
+                phi[(size_t)(t.J + 1) + (size_t)J2 * ((k + 1) + (size_t)K2 * lo)] = out(t.J + 1, k + 1, lo, ph);
             }
-            red[l] = ph;
-            phi[(size_t)(t.J + 1) + (size_t)J2 * ((k + 1) + (size_t)K2 * l)] = out(t.J + 1, k + 1, l, ph);
-            phi[(size_t)(t.J + 1) + (size_t)J2 * ((k + 1) + (size_t)K2 * (l + lm))] = out(t.J + 1, k + 1, l + lm, ph);
         }
         __syncthreads();
         // PHAC(K): the first largest-|ER| deviation, ER = 1 - PH(L)/PHMAX,
@@ -896,40 +929,65 @@ __global__ void __launch_bounds__(128) k_star_rim(DevTables t, BatchPtrs bp, Wor
 //   sum over K = 2..KMAX1, J = JMIN..JMAX1 of THISMASS*COS(PSI_L)*RHF(J)
 //   (and SIN), THISMASS = RHO*RHF(J)*ROF3N*ZOF3N*2*DTHETA,
 // into DIAG[kDiagPart + 2L..].  Grid (L, batch); fixed summation order.
-__global__ void __launch_bounds__(256) k_star_moment(DevTables t, BatchPtrs bp, Work w, StarDev x)
+// HBM-bound (RHO once, after the forward transform has left little of it in
+// L2): a warp takes whole rows K, its lanes consecutive J, eight loads of two
+// rows in flight.  At 256x128x256: 72 us with 256 threads, one load at a time and
+// a division per element, now 17 us (4.0 TB/s).
+constexpr int kMomWarps = 32;
+__global__ void __launch_bounds__(32 * kMomWarps) k_star_moment(DevTables t, BatchPtrs bp, Work w, StarDev x)
 {
     const int l = blockIdx.x, b = blockIdx.y, J2 = t.J + 2, K2 = t.K + 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double *rho = bp.rho[b] + (size_t)J2 * K2 * l;
-    const int j0 = x.jmin - 1, nj = t.J + 1 - j0;   // 0-based J = JMIN-1 .. JMAX
+    const int j0 = x.jmin - 1;   // 0-based J = JMIN-1 .. JMAX
     const double c = t.cosm[l], s = t.sinm[l];
     double sx = 0.0, sy = 0.0;
-    if (nj > 0) {
-        for (int i = threadIdx.x; i < nj * t.K; i += blockDim.x) {
-            const int j = j0 + i % nj, k = 1 + i / nj;
-            const double r = t.rhf[j];
-            double m = __dmul_rn(rho[(size_t)j + (size_t)J2 * k], r);
-            m = __dmul_rn(m, x.rof3n);
-            m = __dmul_rn(m, x.zof3n);
-            m = __dmul_rn(m, 2.0);
-            m = __dmul_rn(m, x.dtheta);
-            sx = __dadd_rn(sx, __dmul_rn(__dmul_rn(m, c), r));
-            sy = __dadd_rn(sy, __dmul_rn(__dmul_rn(m, s), r));
+    constexpr int U = 4;
+    for (int jb = j0 + lane; jb <= t.J; jb += 32 * U) {
+        double r[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) r[u] = jb + 32 * u <= t.J ? __ldg(t.rhf + jb + 32 * u) : 0.0;
+        for (int k = 1 + warp; k <= t.K; k += 2 * kMomWarps) {
+            double v[2][U];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int kk = k + h * kMomWarps, j = jb + 32 * u;
+                    v[h][u] = kk <= t.K && j <= t.J ? __ldg(rho + (size_t)j + (size_t)J2 * kk) : 0.0;
+                }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    double m = __dmul_rn(v[h][u], r[u]);
+                    m = __dmul_rn(m, x.rof3n);
+                    m = __dmul_rn(m, x.zof3n);
+                    m = __dmul_rn(m, 2.0);
+                    m = __dmul_rn(m, x.dtheta);
+                    sx = __dadd_rn(sx, __dmul_rn(__dmul_rn(m, c), r[u]));
+                    sy = __dadd_rn(sy, __dmul_rn(__dmul_rn(m, s), r[u]));
+                }
         }
     }
-    __shared__ double part[2][8];
+    __shared__ double part[2][kMomWarps];
     for (int o = 16; o > 0; o >>= 1) {
         sx += __shfl_xor_sync(0xffffffffu, sx, o);
         sy += __shfl_xor_sync(0xffffffffu, sy, o);
     }
-    const int wp = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) { part[0][wp] = sx; part[1][wp] = sy; }
+    if (lane == 0) { part[0][warp] = sx; part[1][warp] = sy; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double ax = 0.0, ay = 0.0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); i++) { ax += part[0][i]; ay += part[1][i]; }
-        double *d = w.diag + (size_t)b * w.sdiag + kDiagPart + 2 * l;
-        d[0] = ax;
-        d[1] = ay;
+    if (threadIdx.x < 32) {
+        double ax = part[0][lane], ay = part[1][lane];
+        for (int o = 16; o > 0; o >>= 1) {
+            ax += __shfl_xor_sync(0xffffffffu, ax, o);
+            ay += __shfl_xor_sync(0xffffffffu, ay, o);
+        }
+        if (lane == 0) {
+            double *d = w.diag + (size_t)b * w.sdiag + kDiagPart + 2 * l;
+            d[0] = ax;
+            d[1] = ay;
+        }
     }
 }
 
@@ -965,18 +1023,30 @@ __global__ void __launch_bounds__(128) k_star_fill(DevTables t, Work w, StarDev 
         out[(size_t)j + (size_t)J2 * ((size_t)k + (size_t)K2 * l)] = star_phi(t, x, ix, iy, j, k, l);
 }
 
-// PHICHK / KLOCAT (pot/pot3.f:391-399) and TMASS (pot/boundary.f:554).
-__global__ void k_diag(DevTables t, Work w)
+// PHICHK / KLOCAT (pot/pot3.f:391-399: the first of the largest |PHAC(K)|) and
+// TMASS (pot/boundary.f:554).  One warp per solve; a lane's own candidates and
+// the lanes' are compared by (|value|, earlier K), the serial loop's choice.
+// (By one thread's serial loads: 9.2 us at KMAX = 128, now 3.2 us.)
+__global__ void __launch_bounds__(32) k_diag(DevTables t, Work w)
 {
-    const int b = blockIdx.x;
-    if (threadIdx.x != 0) return;
+    const int b = blockIdx.x, lane = threadIdx.x;
     const double *phac = w.phac + (size_t)b * w.sphac;
     double err = 0.0;
     int klocat = 0;
-    for (int k = 2; k <= t.K + 1; ++k) {
-        const double xx = fabs(phac[k]);
-        if (xx > fabs(err)) { err = phac[k]; klocat = k; }
+    for (int k0 = 2; k0 <= t.K + 1; k0 += 128) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = k0 + 32 * u + lane <= t.K + 1 ? phac[k0 + 32 * u + lane] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (fabs(v[u]) > fabs(err)) { err = v[u]; klocat = k0 + 32 * u + lane; }
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, err, o);
+        const int vk = __shfl_xor_sync(0xffffffffu, klocat, o);
+        if (fabs(v) > fabs(err) || (fabs(v) == fabs(err) && vk != 0 && vk < klocat)) { err = v; klocat = vk; }
+    }
+    if (lane != 0) return;
     double *d = w.diag + (size_t)b * w.sdiag;
     const double *scan = w.scan + (size_t)b * w.sscan;
     d[0] = scan[(size_t)t.nsub * 2 * t.ncol + 0];   // column 0 = TERM(1)*SUMASS, inside sum over all rings
@@ -1041,7 +1111,8 @@ static cudaError_t inverse_l(const DevTables &t, const BatchPtrs &bp, const Work
                              cudaStream_t s, int *launches)
 {
     using T = Tile<L>;
-    const size_t sm = (size_t)T::ROWSI * T::TC * sizeof(double) + (size_t)(L / 2) * 8 + fft_table_bytes<L>() + 16;
+    const size_t sm = (size_t)T::ROWSI * T::TC * sizeof(double) + (size_t)(L / 2) * 8 + fft_table_bytes<L>() + 16 +
+                      4 * 81 * sizeof(double);   // the weights of NPOINT <= 10
     cudaError_t e = ensure_smem((const void *)k_inverse<L>, sm);
     if (e != cudaSuccess) return e;
     // X rows through a tensor map when JMAX is even (16-byte strides), else
@@ -1107,7 +1178,7 @@ cudaError_t launch_inverse(const DevTables &t, const BatchPtrs &bp, const Work &
 cudaError_t launch_star_shift(const DevTables &t, const BatchPtrs &bp, const Work &w, const StarDev &x, int nb,
                               cudaStream_t s)
 {
-    k_star_moment<<<dim3(t.L, nb), 256, 0, s>>>(t, bp, w, x);
+    k_star_moment<<<dim3(t.L, nb), 32 * kMomWarps, 0, s>>>(t, bp, w, x);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_star_shift<<<nb, 32, 0, s>>>(t, w, x);

@@ -594,6 +594,8 @@ int build_host_plan(const chy_grid &g, HostPlan &hp, std::string &err)
         }
     }
     hp.ncol = (int)hp.col_term.size();
+    hp.term_col.assign(132, -1);
+    for (int i = 0; i < hp.ncol; i++) hp.term_col[hp.col_part[i] * 66 + hp.col_term[i]] = i;
 
     // boundary points: top edge then outer edge (pot/boundary.f:50-79)
     {
@@ -756,6 +758,24 @@ int build_host_plan(const chy_grid &g, HostPlan &hp, std::string &err)
             hp.zx[num - (j - 2)] = -RHF(j);
         }
         if (ichk == 1) hp.zx[num + num + 1] = RHF(num + 2);
+        // ZAXPHI's steps (pot/pot3.f:366-374), XPOINT = 0
+        hp.zw.assign((size_t)(np - 1) * (np - 1) * 4, 0.0);
+        for (int i = 1; i <= np - 1; i++)
+            for (int s = 0; s < np - 1; s++) {
+                double *wt = &hp.zw[((size_t)(i - 1) * (np - 1) + s) * 4];
+                wt[1] = wt[2] = 1.0;
+                if (i + 1 + s > np) continue;
+                const double xinv = 1.0 / hp.zx[i];
+                wt[0] = hp.zx[i + 1 + s] * xinv;
+                wt[1] = wt[0] - 1.0;
+                double z = 1.0 / wt[1], e = std::fma(-wt[1], z, 1.0);
+                if (e < 0.0) {   // z is past 1/b: the next value towards zero
+                    z = std::nextafter(z, 0.0);
+                    e = std::fma(-wt[1], z, 1.0);
+                }
+                wt[2] = z;
+                wt[3] = e * z;
+            }
     }
     return CHY_OK;
 }

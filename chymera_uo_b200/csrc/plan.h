@@ -103,6 +103,11 @@ struct HostPlan {
     // ZAXPHI abscissae X(1..NPOINT)
     int npoint = 8;
     double zx[11] = {};
+    // its step weights, [II = 1..NPOINT-1][JJ-II-1 = 0..NPOINT-2][4]: XRATIO,
+    // the divisor XRATIO - 1 and its reciprocal as an unevaluated sum z + l
+    // (z rounded towards zero); {0, 1, 1, 0} past the table
+    std::vector<double> zw;
+    std::vector<int> term_col;               // [132] column of part * 66 + term, or -1
 };
 
 // Validates the descriptor and fills every table.  Returns a CHY_* status and
