@@ -274,6 +274,7 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     char *D = p->d_tables;
     DevTables &t = p->t;
     t.J = hp.J; t.K = hp.K; t.L = hp.L; t.N = hp.N; t.M = hp.M; t.NZ = hp.NZ;
+    t.JX = precision == CHY_PREC_MIXED ? chy_mixed_x_ld(&hp) : hp.J;
     t.nring = hp.nring; t.nkeep = hp.nkeep; t.njk = hp.njk; t.ncol = hp.ncol;
     t.nsub = (int)hp.sub_start.size() - 1; t.ntrm = hp.ntrm; t.maxtrm = g->maxtrm;
     t.isyma = g->isym < 0 ? -g->isym : g->isym; t.npoint = hp.npoint;
@@ -335,7 +336,7 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     chy_mixed_bind_tables(p, D + o_ext);
 
     // ---- work space
-    const size_t nX = (size_t)hp.L * hp.K * hp.J;
+    const size_t nX = (size_t)hp.L * hp.K * t.JX;
     const size_t nsub = hp.sub_start.size() - 1;
     Work &w = p->w;
     w.sX = nX;
@@ -1114,9 +1115,17 @@ extern "C" long long chy_dbg_work(chy_plan *p, const char *name, double *out, lo
     else if (n == "phac") { src = p->w.phac; cnt = p->w.sphac; }
     else if (n == "diag") { src = p->w.diag; cnt = p->w.sdiag; }
     else return -CHY_ERR_ARG;
-    if ((long long)cnt > cap) cnt = (size_t)cap;
     cudaError_t e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemcpy(out, src, cnt * sizeof(double), cudaMemcpyDeviceToHost);
+    if (src == p->w.X && p->t.JX != p->t.J) {   // compact rows of J
+        const size_t J = (size_t)p->t.J, rows = std::min((size_t)p->t.L * p->t.K, (size_t)cap / J);
+        cnt = rows * J;
+        if (e == cudaSuccess)
+            e = cudaMemcpy2D(out, J * sizeof(double), src, (size_t)p->t.JX * sizeof(double), J * sizeof(double), rows,
+                             cudaMemcpyDeviceToHost);
+    } else {
+        if ((long long)cnt > cap) cnt = (size_t)cap;
+        if (e == cudaSuccess) e = cudaMemcpy(out, src, cnt * sizeof(double), cudaMemcpyDeviceToHost);
+    }
     if (e != cudaSuccess) return -cuda_fail(e, "chy_dbg_work");
     return (long long)cnt;
 }

@@ -2,7 +2,9 @@
 // the kernels (internal to libchy_pot3).
 //
 // HBM layout of one solve's work space:
-//   X    [L][K][J]   FP64  azimuthal mode coefficients.  X[l][k][j] is mode l of
+//   X    [L][K][JX]  FP64  azimuthal mode coefficients; JX = J, but J rounded up to
+//                          a multiple of 16 where the fused mixed mode solve needs
+//                          aligned rows (the columns past J hold zero).  X[l][k][j] is mode l of
 //                          PHI(J=j+2, K=k+2): j < J-1, k < K-1 is the interior
 //                          (the unknowns of the mode solve), j = J-1 the outer
 //                          boundary column, k = K-1 the top boundary row.
@@ -65,6 +67,7 @@ struct BlkDev {
 };
 
 struct DevTables {
+    int JX;                         // leading dimension of X, >= J
     int J, K, L, N, M, NZ, nring, nkeep, njk, ncol, nsub, ntrm, maxtrm, isyma, npoint;
     double sf1, pig4, grav, F1, cmmax, ammin, cnmax;
     FftDev fwd, inv;

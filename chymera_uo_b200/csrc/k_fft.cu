@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(256) k_forward(DevTables t, BatchPtrs bp, Work
     // independent, and each row is read by exactly one pair.
     double *X = w.X + (size_t)b * w.sX;
     constexpr int n = T::N, nh = n / 2 + 1;
-    const size_t pl = (size_t)t.K * t.J;
+    const size_t pl = (size_t)t.K * t.JX;
 #pragma unroll
     for (int it = 0; it < (nh * T::TC + 255) / 256; ++it) {
         const int i = threadIdx.x + 256 * it;
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(256) k_forward(DevTables t, BatchPtrs bp, Work
         const double aa = aj + ak, ab = aj - ak, ba = bj + bk, bb = bj - bk;
         const double re = cn * ba + sn * ab, im = sn * ba - cn * ab;
         if (j < t.M) {
-            double *xc = X + (size_t)k * t.J + j;
+            double *xc = X + (size_t)k * t.JX + j;
             xc[(size_t)jp * pl] = (aa + re) * t.sf1;
             if (jp != kp) xc[(size_t)kp * pl] = (aa - re) * t.sf1;
             if (jp >= 1) xc[(size_t)(n + jp) * pl] = (im + bb) * t.sf1;
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(256) k_bdy_synth(DevTables t, Work w)
                 double v = 0.0;
 #pragma unroll
                 for (int p = 0; p < 21; ++p) v = __fma_rn(cq[c][p], f[p], v);
-                X[((size_t)l * t.K + t.jk_k[q]) * t.J + t.jk_j[q]] = v;
+                X[((size_t)l * t.K + t.jk_k[q]) * t.JX + t.jk_j[q]] = v;
             }
         }
         l += blockDim.x;
@@ -613,7 +613,7 @@ __global__ void k_coef(DevTables t, Work w)
     const int j = blockIdx.x * 32 + threadIdx.x, k = blockIdx.y, n = t.N;
     if (j >= t.J) return;
     const double pi = 3.1415926535897932, inv = 1.0 / t.sf1;
-    const size_t pl = (size_t)t.K * t.J, col = (size_t)k * t.J + j;
+    const size_t pl = (size_t)t.K * t.JX, col = (size_t)k * t.JX + j;
     const int J2 = t.J + 2, K2 = t.K + 2;
     const size_t ldl = (size_t)J2 * K2, ldi = ldl * (t.L / 2), off = (size_t)(j + 1) + (size_t)J2 * (k + 1);
     const double a1 = w.X[col] * inv, x1 = fabs(a1);
@@ -790,13 +790,13 @@ __global__ void __launch_bounds__(256) k_inverse(DevTables t, BatchPtrs bp, Work
     if (xmode == 2) {
         // copies issued above
     } else if (xmode == 1) {
-        // JMAX even: 16-byte granules (columns j, j+1 both in range or both
-        // out), aligned since X, JMAX and j0 are
+        // JX even: 16-byte granules (columns j, j+1 both within JX), aligned
+        // since X, JX and j0 are
         constexpr int NG = T::TC / 2;
         for (int i = threadIdx.x; i < (n + 1) * NG; i += blockDim.x) {
             const int g = i % NG, q = i / NG, j = j0 + 2 * g;
             const bool ok = j < t.J, okim = ok && q >= 1 && q < n;
-            const size_t col = (size_t)k * t.J + j, pl = (size_t)t.K * t.J;
+            const size_t col = (size_t)k * t.JX + j, pl = (size_t)t.K * t.JX;
             cp_async16(A + q * RS + 2 * g, ok ? X + (size_t)q * pl + col : X, ok ? 16 : 0);
             cp_async16(A + (I0 + q) * RS + 2 * g, okim ? X + (size_t)(n + q) * pl + col : X, okim ? 16 : 0);
         }
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(256) k_inverse(DevTables t, BatchPtrs bp, Work
         for (int i = threadIdx.x; i < (n + 1) * T::TC; i += blockDim.x) {
             const int c = i % T::TC, q = i / T::TC, j = j0 + c;
             const bool ok = j < t.J, okim = ok && q >= 1 && q < n;
-            const size_t col = (size_t)k * t.J + j, pl = (size_t)t.K * t.J;
+            const size_t col = (size_t)k * t.JX + j, pl = (size_t)t.K * t.JX;
             cp_async8(A + q * RS + c, ok ? X + (size_t)q * pl + col : X, ok ? 8 : 0);
             cp_async8(A + (I0 + q) * RS + c, okim ? X + (size_t)(n + q) * pl + col : X, okim ? 8 : 0);
         }
@@ -1115,15 +1115,15 @@ static cudaError_t inverse_l(const DevTables &t, const BatchPtrs &bp, const Work
                       4 * 81 * sizeof(double);   // the weights of NPOINT <= 10
     cudaError_t e = ensure_smem((const void *)k_inverse<L>, sm);
     if (e != cudaSuccess) return e;
-    // X rows through a tensor map when JMAX is even (16-byte strides), else
+    // X rows through a tensor map when JX is even (16-byte strides), else
     // 8-byte copies
-    int xmode = (t.J & 1) == 0 ? 1 : 0;
+    int xmode = (t.JX & 1) == 0 ? 1 : 0;
     CUtensorMap xmap;
     std::memset(&xmap, 0, sizeof xmap);
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
     if (xmode == 1 && enc && reinterpret_cast<uintptr_t>(w.X) % 16 == 0) {
         const cuuint64_t dims[3] = {(cuuint64_t)t.J, (cuuint64_t)t.K, (cuuint64_t)L * nb};
-        const cuuint64_t strides[2] = {(cuuint64_t)t.J * 8, (cuuint64_t)t.J * t.K * 8};
+        const cuuint64_t strides[2] = {(cuuint64_t)t.JX * 8, (cuuint64_t)t.JX * t.K * 8};
         const cuuint32_t box[3] = {(cuuint32_t)T::TC, 1u, (cuuint32_t)(T::N < 256 ? T::N : 256)}, es[3] = {1, 1, 1};
         if (enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, w.X, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,

@@ -95,8 +95,8 @@ struct MixedDev {
                                 // polls on a barrier nothing arrives on (0: off)
 };
 
-// Arrays of the multi-kernel mixed pipeline (grids with JMAX > 256 or JMAX
-// not a multiple of 16).  item = solve * L + mode; Jt = JMAX rounded up to a
+// Arrays of the multi-kernel mixed pipeline (grids with JMAX > 256 or JMAX = 1
+// mod 16).  item = solve * L + mode; Jt = JMAX rounded up to a
 // multiple of 256 (the GEMM N tile).
 struct WideDev {
     double *xit;                // [item][K][J] FP64 iterate
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_mixed(DevTables t, Work w, Mixe
 {
     extern __shared__ __align__(1024) uint8_t sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int NT = x.ntile, M = t.M, NZ = t.NZ, J = t.J, K = t.K;
+    const int NT = x.ntile, M = t.M, NZ = t.NZ, J = t.JX, K = t.K;
     uint8_t *sA = sm + MixedSmem::a;
     uint8_t *sBh = sm + MixedSmem::b, *sBl = sBh + (size_t)NT * 256;
     double *d_am = reinterpret_cast<double *>(sm + MixedSmem::tables(NT));   // [256]
@@ -632,9 +632,9 @@ __global__ void __launch_bounds__(256, 1) k_mode_mixed(DevTables t, Work w, Mixe
             float sxf0 = 0.f, sxf1 = 0.f;               // kRes: sums of x0^2 per half (unscaled)
             // ---- residual r = Y - A_m x (FP64) -> TMEM cols [256, 256+NT) as FP32.
             // Out-of-range neighbours read as 0; their stencil coefficients
-            // (AN(1), CN(KMAX-1), AM(1), CM(JMAX-1)) are 0 too.  JMAX is a
-            // multiple of 16, so column M is in the chunk of column M-1 and
-            // every 16-byte granule of a row is aligned.
+            // (AN(1), CN(KMAX-1), AM(1), CM(JMAX-1)) are 0 too.  JX is a
+            // multiple of 16 and M is not, so column M is in the tile of
+            // column M-1 and every 16-byte granule of a row is aligned.
             float rmax0 = 0.0f, rmax1 = 0.0f;           // max |r| per half
             if constexpr (kRes) {
                 // Raw X rows k = 0..KMAX-1 (boundary row NZ and column M
@@ -1348,7 +1348,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_pair(DevTables t, Work w, Mixed
     const int g = warp >> 2, gt = tid & 127;            // group, thread in group
     const uint32_t rank = cluster_rank(), peer = rank ^ 1u;
     const int NT = x.ntile, NH = NT / 2, col0 = (int)rank * NH;
-    const int M = t.M, NZ = t.NZ, J = t.J, K = t.K;
+    const int M = t.M, NZ = t.NZ, J = t.JX, K = t.K;
     uint8_t *sA = sm + PairSmem::a;
     uint8_t *sB = sm + PairSmem::b + (size_t)g * kPairB;
     uint8_t *sBh = sB, *sBl = sB + (size_t)NH * 256;
@@ -1926,8 +1926,8 @@ __global__ void __launch_bounds__(256, 1) k_mode_pair(DevTables t, Work w, Mixed
 
 // ---------------------------------------------------------------------------
 // Wide pipeline: grids whose radial extent does not fit one CTA's tiles
-// (JMAX > 256, e.g. the 512 x 128 x 512 serving class) or whose rows are not
-// 16-byte tiles (JMAX not a multiple of 16).  The same refinement as
+// (JMAX > 256, e.g. the 512 x 128 x 512 serving class) or whose boundary column
+// starts a 16-column tile (JMAX = 1 mod 16).  The same refinement as
 // k_mode_mixed -- FP64 residual, FP16 hi/lo tensor-core transforms with FP32
 // accumulation, FP32 radial sweeps from the same sweep table, FP64 update --
 // as five kernels per approximate solve, with the intermediate FP32 arrays in
@@ -2209,8 +2209,13 @@ __global__ void __launch_bounds__(256) k_wide_update(DevTables t, Work w, MixedD
 static int round64(int v) { return (v + 63) / 64 * 64; }
 
 // Grids the single-kernel mode solve covers; the others take the wide
-// pipeline.
-static bool mixed_fused(const chy::HostPlan *hp) { return hp->J % 16 == 0 && round64(hp->J) <= kMaxN; }
+// pipeline.  Its tiles are 16 columns wide, aligned, and hold the boundary
+// column M = JMAX-1 beside column M-1: rows of X are padded to a multiple of 16
+// columns, and only JMAX = 1 mod 16 (M the first column of a tile) stays out.
+// Four solves of 189x64x128: 0.89 ms by the wide pipeline, 0.30 ms fused.
+static bool mixed_fused(const chy::HostPlan *hp) { return hp->J % 16 != 1 && round64(hp->J) <= kMaxN; }
+
+int chy_mixed_x_ld(const chy::HostPlan *hp) { return mixed_fused(hp) ? (hp->J + 15) / 16 * 16 : hp->J; }
 
 bool chy_mixed_supported(const chy::HostPlan *hp)
 {
@@ -2374,7 +2379,7 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
     if (!p->mx) p->mx = new MixedState();
     MixedDev &d = p->mx->dev;
     const chy::HostPlan &hp = p->hp;
-    d.sxb = (size_t)hp.L * hp.K * hp.J;
+    d.sxb = (size_t)hp.L * hp.K * p->t.JX;
     d.scorr = (size_t)hp.L * 16;
     d.xbuf = nullptr;
     d.corr = base;
@@ -2403,11 +2408,11 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
         cudaMallocHost(&p->mx->h_corr, sizeof(double) * d.scorr * p->max_batch);
         cudaMallocHost(&p->mx->h_err, sizeof(int));
         // the residual's right-hand-side tiles: X viewed as max_batch*L*K rows
-        // of J doubles; one item is K consecutive rows
+        // of JX doubles; one item is K consecutive rows
         PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-        if (enc && hp.K <= 256 && hp.J % 16 == 0) {
-            const cuuint64_t dims[2] = {(cuuint64_t)hp.J, (cuuint64_t)p->max_batch * hp.L * hp.K};
-            const cuuint64_t strides[1] = {(cuuint64_t)hp.J * sizeof(double)};
+        if (enc && hp.K <= 256 && p->t.JX % 16 == 0) {
+            const cuuint64_t dims[2] = {(cuuint64_t)p->t.JX, (cuuint64_t)p->max_batch * hp.L * hp.K};
+            const cuuint64_t strides[1] = {(cuuint64_t)p->t.JX * sizeof(double)};
             const cuuint32_t box[2] = {16, (cuuint32_t)hp.K}, box_s[2] = {16, (cuuint32_t)(hp.K - 1)};
             const cuuint32_t es[2] = {1, 1};
             p->mx->tm_ok = enc(&p->mx->tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, p->w.X, dims, strides, box, es,
@@ -2469,7 +2474,7 @@ int chy_mixed_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
     if (d.nit > 8) d.nit = 8;
     if (d.nit > 2 && !d.xbuf) return CHY_ERR_NOT_SETUP;
     // the kernel streams X and the iterate with 16-byte async copies
-    if ((reinterpret_cast<uintptr_t>(p->w.X) | reinterpret_cast<uintptr_t>(d.xbuf)) % 16 != 0 || p->hp.J % 16 != 0)
+    if ((reinterpret_cast<uintptr_t>(p->w.X) | reinterpret_cast<uintptr_t>(d.xbuf)) % 16 != 0 || p->t.JX % 16 != 0)
         return CHY_ERR_ARG;
     const size_t sm = MixedSmem::bytes(d.ntile);
     // two approximate solves (one correction) keep the iterate in tensor memory

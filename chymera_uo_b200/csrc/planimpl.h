@@ -128,6 +128,8 @@ size_t chy_internal_drop_blk_table(chy_plan *p);
 
 // Mixed-precision mode solve (k_mixed.cu).
 bool chy_mixed_supported(const chy::HostPlan *hp);
+// Leading dimension of X in a mixed plan.
+int chy_mixed_x_ld(const chy::HostPlan *hp);
 // Appends the mixed path's tables to the packed table image; returns offset.
 size_t chy_mixed_pack_tables(const chy::HostPlan *hp, std::vector<char> *image, bool mixed);
 void chy_mixed_bind_tables(chy_plan *p, char *dev_base);
