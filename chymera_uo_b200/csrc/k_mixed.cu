@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "planimpl.h"
@@ -86,7 +87,7 @@ struct MixedDev {
     const float *sw_piv;        // [N+1][ntile][128] pivot reciprocals 1/D
     double *xbuf;               // [nb][L][K][J] FP64 iterate
     size_t sxb;
-    double *corr;               // [nb][L][8][2] per mode: sum delta^2, sum x^2
+    double *corr;               // [nb][L][8][2] per mode (wide: per mode and tile): sum delta^2, sum x^2
     size_t scorr;
     int *err;                   // error word
     int nit;                    // approximate solves (1 + corrections)
@@ -96,22 +97,20 @@ struct MixedDev {
 };
 
 // Arrays of the multi-kernel mixed pipeline (grids with JMAX > 256 or JMAX = 1
-// mod 16).  item = solve * L + mode; Jt = JMAX rounded up to a
-// multiple of 256 (the GEMM N tile).
+// mod 16).  item = solve * L + mode; nt = ceil(JMAX / 64) tiles of 64 columns.
 struct WideDev {
-    double *xit;                // [item][K][J] FP64 iterate
-    size_t sxit;
-    float *R;                   // [item][Jt][128] FP32: residual rows, then the sweep results
-    float *O;                   // [item][Jt][128] FP32: products U r (W) and V w (delta)
-    size_t sro;
-    unsigned *rmax, *wmax;      // [item][Jt/256] bits of max |r| and max |w| per tile
-    int Jt, nt;                 // nt = Jt / 256
+    float *W;                   // [item][64 nt][128]: products U r, swept in place to w
+    size_t sw;
+    float *F;                   // [item][KMAX-1][J]: the first solution, x0 = F / d_k
+    double *xit;                // [item][KMAX-1][J] FP64 iterate (two or more corrections)
+    size_t sx;
+    int nt;
 };
 
 struct MixedState {
     size_t o_aimg = 0, o_lam = 0;   // offsets into the packed table image
     MixedDev dev{};
-    double *h_corr = nullptr;       // pinned [max_batch][L][8][2]
+    double *h_corr = nullptr;       // pinned copy of corr
     size_t xbuf_bytes = 0;          // FP64 iterate (two or more corrections)
     int *h_err = nullptr;           // pinned
     int probe_polls = 0;            // test hook (chy_dbg_mixed_probe)
@@ -1930,276 +1929,540 @@ __global__ void __launch_bounds__(256, 1) k_mode_pair(DevTables t, Work w, Mixed
 // starts a 16-column tile (JMAX = 1 mod 16).  The same refinement as
 // k_mode_mixed -- FP64 residual, FP16 hi/lo tensor-core transforms with FP32
 // accumulation, FP32 radial sweeps from the same sweep table, FP64 update --
-// as five kernels per approximate solve, with the intermediate FP32 arrays in
-// device memory:
-//   k_wide_resid   r = Y - A x (FP64) -> R[item][j][k] (FP32), per-tile max |r|
-//   k_wide_gemm    W = U r: one CTA per (item, 256-column tile), tcgen05
-//   k_wide_sweep   (T_r(m) + lam_p) w = W_p, one thread per (item, p) -> R
-//   k_wide_gemm    delta = V w
-//   k_wide_update  x += delta (FP64); the last solve writes X's interior
+// as three kernels per approximate solve, with FP32 arrays in device memory
+// between them:
+//   k_wide_down    r = Y - A x (FP64), W = U r: 64-column tiles, tcgen05
+//   k_wide_sweep   (T_r(m) + lam_p) w = W_p, two threads per (item, p), in place
+//   k_wide_up      delta = V w by tcgen05, x += delta (FP64); the last solve
+//                  writes X's interior
+// The residual is formed in the registers that split it into the product's
+// operand, and the update in the product's epilogue, so neither passes through
+// memory.  The first solution is an FP32 accumulator times a power of two and
+// 1/d_k, so its FP32 part F holds it exactly and takes half an FP64 iterate's
+// bytes.  Bound by HBM: 11.4 GB at four solves of 512x128x512 with one
+// correction (1.75 ms at the measured rate).  Measured there, all mode solves:
+// five kernels with residual, scaled rows and update each through memory 6.35
+// ms, now 3.27 (down 0.51 and 1.10, sweeps 0.36 each, up 0.41 and 0.52).  What is
+// left is latency at 16 warps per SM: two CTAs fill registers and shared memory.
 // ---------------------------------------------------------------------------
-constexpr int kWideN = 256;      // GEMM N tile (radial columns)
 constexpr int kWideMaxJ = 1024;  // largest JMAX of the wide pipeline
-constexpr int kWideTiles = kWideMaxJ / kWideN;
+constexpr int kWideT = 64;       // columns of a tile: two CTAs per SM, one loading while the other multiplies
 
-template <bool kFirst>
-__global__ void __launch_bounds__(256) k_wide_resid(DevTables t, Work w, MixedDev x, WideDev d, int nb)
-{
-    __shared__ float tile[32][129];
-    __shared__ float red[8];
-    const int item = blockIdx.y, b = item / t.L, l = item % t.L, j0 = blockIdx.x * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, j = j0 + tx;
-    const int M = t.M, NZ = t.NZ, J = t.J;
-    const int m = l <= t.N ? l : l - t.N;
-    const double xl2 = 2.0 * (t.xlamm[m] - 1.0);
-    const double *Xl = w.X + (size_t)b * w.sX + (size_t)l * t.K * J;
-    const double *xl = d.xit + (size_t)item * d.sxit;
-    double bmj = 0.0, amj = 0.0, cmj = 0.0;
-    if (j < M) {
-        bmj = t.bm0[j] + xl2 * t.cc[j];
-        if (j == 0) bmj = t.bm0[0] + (((m & 1) ? -1.0 : 1.0) - 1.0) * t.ammin + xl2 * t.cc[0];
-        amj = t.am[j];
-        cmj = t.cm[j];
-    }
-    float vmax = 0.0f;
-    for (int k = ty; k < 128; k += 8) {
-        float v = 0.0f;
-        if (k < NZ && j < M) {
-            // 4 pi G rho with the boundary folds (pot/pot3.f:212-224)
-            double r = t.pig4 * Xl[(size_t)k * J + j];
-            if (k == NZ - 1) r = r - t.cnmax * Xl[(size_t)NZ * J + j];
-            if (j == M - 1) r = r - t.cmmax * Xl[(size_t)k * J + M];
-            if (!kFirst) {
-                const double *xr = xl + (size_t)k * J;
-                double ax = (t.bn[k] + bmj) * xr[j];
-                if (k > 0) ax += t.an[k] * xl[(size_t)(k - 1) * J + j];
-                if (k < NZ - 1) ax += t.cn[k] * xl[(size_t)(k + 1) * J + j];
-                if (j > 0) ax += amj * xr[j - 1];
-                if (j < M - 1) ax += cmj * xr[j + 1];
-                r = r - ax;
-            }
-            v = (float)(x.zsc[k] * r);   // times d_k for the orthogonal transform
-        }
-        tile[tx][k] = v;
-        vmax = fmaxf(vmax, fabsf(v));
-    }
-    __syncthreads();
-    float *Ri = d.R + (size_t)item * d.sro;
-    for (int e = threadIdx.x; e < 32 * 128; e += 256) {
-        const int jj = e >> 7, k = e & 127;
-        Ri[(size_t)(j0 + jj) * 128 + k] = tile[jj][k];
-    }
-    vmax = warp_max(vmax);
-    if ((threadIdx.x & 31) == 0) red[ty] = vmax;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float mx = red[0];
-        for (int i = 1; i < 8; ++i) mx = fmaxf(mx, red[i]);
-        if (mx > 0.0f) atomicMax(d.rmax + (size_t)item * d.nt + j0 / kWideN, __float_as_uint(mx));
-    }
-}
+// Shared memory of the two product kernels: eigenbasis tile, operand tile (then,
+// in k_wide_up, the staged product), row tables, reductions, barriers.
+struct WideSmem {
+    static constexpr int a = 0, b = kAImg, rows = b + kWideT * 512, red = rows + 5 * 128 * 8, bars = red + 32 * 8,
+                         bytes = bars + 64;
+};
 
-// out[item][j][row] = sum_k A(row, k) in[item][j][k] for one 256-column tile:
-// A is the plan's 2^12-scaled FP16 hi/lo image of Q^T, or with trans its
-// transpose Q; the input tile is scaled by a power of two from its maximum
-// and split to FP16 hi/lo in shared memory, three MMA passes accumulate in
-// FP32 in tensor memory.
-__global__ void __launch_bounds__(256, 1) k_wide_gemm(const uint8_t *aimg, const float *in, float *out,
-                                                      const unsigned *tmax, WideDev d, int trans, int *err)
+// Per-CTA state of a product kernel: tensor memory (64 columns), barriers, the
+// eigenbasis tile on its way, and per row k {BN, d_k AN_k / d_(k-1)},
+// {d_k CN_k / d_(k+1), d_k} and 1/d_k.
+struct WideCta {
+    uint8_t *sA, *sBh, *sBl;
+    double2 *ba, *cd;
+    double *ek;
+    float *red;
+    uint64_t *bars;     // [0] product, [1] eigenbasis tile
+    uint32_t *slot;
+    int *flag;
+    uint32_t tmem, ph;
+    bool a_wait, failed;
+};
+
+__device__ __forceinline__ void wide_setup(WideCta &c, uint8_t *sm, const DevTables &t, const MixedDev &x)
 {
-    extern __shared__ __align__(1024) uint8_t sm[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tile = blockIdx.x, item = blockIdx.y;
-    uint8_t *sA = sm, *sBh = sm + kAImg, *sBl = sBh + (size_t)kWideN * 256;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sBl + (size_t)kWideN * 256);   // [0] product, [1] A tile
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2);
-    int *flag = reinterpret_cast<int *>(slot + 1);
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(slot)));
+    const int tid = threadIdx.x;
+    c.sA = sm + WideSmem::a;
+    c.sBh = sm + WideSmem::b;
+    c.sBl = c.sBh + kWideT * 256;
+    c.ba = reinterpret_cast<double2 *>(sm + WideSmem::rows);
+    c.cd = c.ba + 128;
+    c.ek = reinterpret_cast<double *>(c.cd + 128);
+    c.red = reinterpret_cast<float *>(sm + WideSmem::red);
+    c.bars = reinterpret_cast<uint64_t *>(sm + WideSmem::bars);
+    c.slot = reinterpret_cast<uint32_t *>(c.bars + 2);
+    c.flag = reinterpret_cast<int *>(c.slot + 1);
+    if (tid < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(smem_u32(c.slot)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        *flag = 0;
+        mbar_init(&c.bars[0], 1);
+        mbar_init(&c.bars[1], 1);
+        *c.flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        mbar_expect_tx(&bars[1], kAImg);
-        bulk_g2s(sA, aimg, kAImg, &bars[1]);
+        mbar_expect_tx(&c.bars[1], kAImg);
+        bulk_g2s(c.sA, x.aimg, kAImg, &c.bars[1]);
     }
-    const float s = pow2_scale(__uint_as_float(tmax[(size_t)item * d.nt + tile]));
-    // the tile's rows as 16-byte loads, eight in flight per thread
-    const float4 *src = reinterpret_cast<const float4 *>(in + (size_t)item * d.sro + (size_t)tile * kWideN * 128);
-#pragma unroll 8
-    for (int i = tid; i < kWideN * 32; i += 256) {
-        const float4 v = src[i];
-        const int row = i >> 5, k = (i & 31) * 4;
-        put_split(sBh, sBl, row, k, kWideN, v.x * s);
-        put_split(sBh, sBl, row, k + 1, kWideN, v.y * s);
-        put_split(sBh, sBl, row, k + 2, kWideN, v.z * s);
-        put_split(sBh, sBl, row, k + 3, kWideN, v.w * s);
+    for (int k = tid; k < 128; k += blockDim.x) {
+        c.ba[k] = make_double2(k < t.NZ ? t.bn[k] : 0.0, x.zsc[256 + k]);
+        c.cd[k] = make_double2(x.zsc[384 + k], x.zsc[k]);
+        c.ek[k] = x.zsc[128 + k];
     }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    c.tmem = *c.slot;
+    c.ph = 0;
+    c.a_wait = true;
+    c.failed = false;
+}
+
+// Largest |v| of the block, known to every thread (one barrier).
+__device__ __forceinline__ float wide_max(const WideCta &c, float v)
+{
+    v = warp_max(v);
+    if ((threadIdx.x & 31) == 0) c.red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float m = c.red[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) m = fmaxf(m, c.red[i]);
+    return m;
+}
+
+// The tile's product once its operand is in shared memory (every thread has
+// written its part): false after a wait that ran out, then for good.
+__device__ __forceinline__ bool wide_product(WideCta &c, bool trans)
+{
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *slot;
-    // the A tile: every thread waits (bounded); a phase counts only if all saw it
-    bool a_ok = mbar_wait(&bars[1], 0);
-    if (!a_ok) *flag = 1;
-    __syncthreads();
-    a_ok = *flag == 0;
-    const uint32_t idesc = (1u << 4) | ((uint32_t)(kWideN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-    if (a_ok && tid == 0) gemm_issue(tmem, sA, sBh, kWideN, idesc, &bars[0], trans != 0);
-    bool d_ok = a_ok && mbar_wait(&bars[0], 0);
-    if (a_ok && !d_ok) *flag = 1;
-    __syncthreads();
-    d_ok = *flag == 0;
-    tc_fence_after();
-    float *dst = out + (size_t)item * d.sro + (size_t)tile * kWideN * 128;
-    const int q = warp & 3, row = 32 * q + lane;
-    if (d_ok) {
-        const float unscale = 1.0f / (kAScale * s);
-        for (int c0 = (warp >> 2) * 128; c0 < (warp >> 2) * 128 + 128; c0 += 32) {
-            float v[32];
-            tm_ld32(tmem + ((uint32_t)(32 * q) << 16) + c0, v);
-#pragma unroll
-            for (int u = 0; u < 32; ++u) dst[(size_t)(c0 + u) * 128 + row] = v[u] * unscale;
-        }
-    } else {
-        // drain (bounded) what is still in flight, then make the tile NaN so the
-        // failure reaches PHI, and raise the error word
-        if (!a_ok) mbar_wait(&bars[1], 0);
-        else mbar_wait(&bars[0], 0);
-        for (int c0 = (warp >> 2) * 128; c0 < (warp >> 2) * 128 + 128; ++c0) dst[(size_t)c0 * 128 + row] = __int_as_float(0x7fc00000);
-        if (tid == 0) atomicExch(err, 1);
+    if (c.failed) return false;
+    bool ok = true;
+    if (c.a_wait) {   // the eigenbasis tile, before the first product
+        ok = mbar_wait(&c.bars[1], 0);
+        if (!ok) *c.flag = 1;
+        __syncthreads();
+        ok = *c.flag == 0;
+        c.a_wait = !ok;
     }
+    const uint32_t idesc = (1u << 4) | ((uint32_t)(kWideT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    if (ok) {
+        if (threadIdx.x == 0) gemm_issue(c.tmem, c.sA, c.sBh, kWideT, idesc, &c.bars[0], trans);
+        if (!mbar_wait(&c.bars[0], c.ph)) *c.flag = 1;
+        __syncthreads();
+        ok = *c.flag == 0;
+        if (ok) c.ph ^= 1u;
+        else mbar_wait(&c.bars[0], c.ph);   // drain (bounded) what is still in flight
+    } else {
+        mbar_wait(&c.bars[1], 0);
+    }
+    tc_fence_after();
+    c.failed = !ok;
+    return ok;
+}
+
+__device__ __forceinline__ void wide_release(const WideCta &c, int *err)
+{
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
+    if (threadIdx.x == 0 && c.failed) atomicExch(err, 1);
+    if (threadIdx.x == 0 && c.a_wait && !c.failed) mbar_wait(&c.bars[1], 0);   // a CTA without a tile
+    __syncthreads();
+    if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(c.tmem));
 }
 
-// (T_r(m) + lam_p) w = W_p for each p (thread) of one item (block), with the
-// sweep table's pivot reciprocals and multipliers: rows [0, h) top-down,
-// [h, M) bottom-up, meeting at rows h-1 and h -- k_mode_mixed's sweeps on
-// CUDA cores.  W comes from O, w goes to R (zero past M and for p >= NZ).
-__global__ void __launch_bounds__(128) k_wide_sweep(DevTables t, MixedDev x, WideDev d)
+// One 128-byte line on its way into L2: a tile's loads then wait for L2, not HBM.
+__device__ __forceinline__ void l2_prefetch(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// `bytes` (a multiple of 16) from p, likewise.
+__device__ __forceinline__ void l2_prefetch_bulk(const void *p, uint32_t bytes)
 {
-    extern __shared__ float s_tab[];   // AM, CM as FP32 (M each)
-    float *s_am = s_tab, *s_cm = s_tab + t.M;
-    __shared__ float red[4][kWideTiles];
-    const int item = blockIdx.x, l = item % t.L, p = threadIdx.x, M = t.M;
-    const int m = l <= t.N ? l : l - t.N;
-    const int NTs = x.ntile, h = 32 * ((M + 63) / 64);
-    for (int j = threadIdx.x; j < M; j += blockDim.x) {
-        s_am[j] = (float)t.am[j];
-        s_cm[j] = (float)t.cm[j];
-    }
-    __syncthreads();
-    const float *W = d.O + (size_t)item * d.sro + p;
-    float *wo = d.R + (size_t)item * d.sro + p;
-    const float *piv = x.sw_piv + (size_t)m * NTs * 128 + p, *mul = x.sw_mul + (size_t)m * NTs * 128 + p;
-    float tmx[kWideTiles];
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ uint32_t pack_half2(__half a, __half b)
+{
+    return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
+}
+
+// W[item][j][p] = sum_k U(p,k) r(j,k) for 64-column tiles of every item.  kSrc:
+// the iterate the residual subtracts: 0 none, 1 F / d_k, 2 xit.  Warp w forms
+// rows 16 w .. 16 w + 15 of columns lane and lane + 32: consecutive k, so that a
+// thread's values are whole 16-byte granules of the operand tile.
+template <int kSrc>
+__global__ void __launch_bounds__(256, 2) k_wide_down(DevTables t, Work w, MixedDev x, WideDev d, int tiles)
+{
+    extern __shared__ __align__(1024) uint8_t sm[];
+    WideCta c;
+    wide_setup(c, sm, t, x);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, M = t.M, NZ = t.NZ, J = t.JX, k0 = 16 * warp;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int item = tile / d.nt, j0 = (tile - item * d.nt) * kWideT;
+        const int l = item % t.L, m = l <= t.N ? l : l - t.N;
+        const double xl2 = 2.0 * (t.xlamm[m] - 1.0);
+        const double *Xl = w.X + (size_t)item * t.K * J;   // X's solves are L * K * J apart
+        const float *Fl = d.F + (size_t)item * d.sx;
+        const double *xl = d.xit + (size_t)item * d.sx;
+        if (tile + (int)gridDim.x < tiles) {   // the next tile: KMAX rows of 512 bytes of X, 256 of F
+            const int nt = tile + gridDim.x, ni = nt / d.nt, nj = (nt - ni * d.nt) * kWideT;
+            for (int i = threadIdx.x; i < 4 * t.K; i += 256)
+                if (nj + 16 * (i & 3) < J) l2_prefetch(w.X + ((size_t)ni * t.K + (i >> 2)) * J + nj + 16 * (i & 3));
+            if constexpr (kSrc == 1)
+                for (int i = threadIdx.x; i < 2 * NZ; i += 256)
+                    if (nj + 32 * (i & 1) < M) l2_prefetch(d.F + (size_t)ni * d.sx + (size_t)(i >> 1) * t.J + nj + 32 * (i & 1));
+            if constexpr (kSrc == 2)
+                for (int i = threadIdx.x; i < 4 * NZ; i += 256)
+                    if (nj + 16 * (i & 3) < M) l2_prefetch(d.xit + (size_t)ni * d.sx + (size_t)(i >> 2) * t.J + nj + 16 * (i & 3));
+        }
+        double bm[2], am[2], cm[2];
 #pragma unroll
-    for (int i = 0; i < kWideTiles; ++i) tmx[i] = 0.0f;
-    if (p < t.NZ) {
-        float yp = 0.0f;
-#pragma unroll 8
-        for (int j = 0; j < h; ++j) {
-            const float rr = piv[(size_t)j * 128], ar = s_am[j] * rr;
-            yp = fmaf(-ar, yp, W[(size_t)j * 128] * rr);
-            wo[(size_t)j * 128] = yp;
-        }
-        const float yt = yp;
-        yp = 0.0f;
-#pragma unroll 8
-        for (int j = M - 1; j >= h; --j) {
-            const float rr = piv[(size_t)j * 128], cr = s_cm[j] * rr;
-            yp = fmaf(-cr, yp, W[(size_t)j * 128] * rr);
-            wo[(size_t)j * 128] = yp;
-        }
-        const float yu = yp, et = mul[(size_t)(h - 1) * 128], fu = mul[(size_t)h * 128];
-        const float xt = (yt + (1.0f - et) * yu) / ((et + fu) - et * fu);
-        const float xu = yu + (1.0f - fu) * xt;
-        float xn = xt;
-        wo[(size_t)(h - 1) * 128] = xt;
-        tmx[(h - 1) / kWideN] = fmaxf(tmx[(h - 1) / kWideN], fabsf(xt));
-#pragma unroll 8
-        for (int j = h - 2; j >= 0; --j) {
-            xn = wo[(size_t)j * 128] + (1.0f - mul[(size_t)j * 128]) * xn;
-            wo[(size_t)j * 128] = xn;
-            tmx[j / kWideN] = fmaxf(tmx[j / kWideN], fabsf(xn));
-        }
-        float xp = xu;
-        wo[(size_t)h * 128] = xu;
-        tmx[h / kWideN] = fmaxf(tmx[h / kWideN], fabsf(xu));
-#pragma unroll 8
-        for (int j = h + 1; j < M; ++j) {
-            xp = wo[(size_t)j * 128] + (1.0f - mul[(size_t)j * 128]) * xp;
-            wo[(size_t)j * 128] = xp;
-            tmx[j / kWideN] = fmaxf(tmx[j / kWideN], fabsf(xp));
-        }
-        for (int j = M; j < d.Jt; ++j) wo[(size_t)j * 128] = 0.0f;
-    } else {
-        for (int j = 0; j < d.Jt; ++j) wo[(size_t)j * 128] = 0.0f;
-    }
-    for (int i = 0; i < d.nt; ++i) {
-        const float v = warp_max(tmx[i]);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][i] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < d.nt) {
-        const float v = fmaxf(fmaxf(red[0][threadIdx.x], red[1][threadIdx.x]), fmaxf(red[2][threadIdx.x], red[3][threadIdx.x]));
-        if (v > 0.0f) atomicMax(d.wmax + (size_t)item * d.nt + threadIdx.x, __float_as_uint(v));
-    }
-}
-
-// x += delta (FP64) for one item per block; the last solve writes X's
-// interior.  Per-item sums of delta^2 and x^2 go to the correction report.
-__global__ void __launch_bounds__(256) k_wide_update(DevTables t, Work w, MixedDev x, WideDev d, int it, int last)
-{
-    __shared__ float tile[128][33];
-    __shared__ double red[2][8];
-    const int item = blockIdx.x, b = item / t.L, l = item % t.L, M = t.M, NZ = t.NZ, J = t.J;
-    double *Xl = w.X + (size_t)b * w.sX + (size_t)l * t.K * J;
-    double *xl = d.xit + (size_t)item * d.sxit;
-    const float *O = d.O + (size_t)item * d.sro;
-    double sd = 0.0, sx = 0.0;
-    for (int j0 = 0; j0 < M; j0 += 32) {
-        for (int e = threadIdx.x; e < 32 * 128; e += 256) {
-            const int jj = e >> 7, k = e & 127;
-            tile[k][jj] = O[(size_t)(j0 + jj) * 128 + k];
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < 32 * NZ; e += 256) {
-            const int k = e >> 5, jj = e & 31, j = j0 + jj;
+        for (int h = 0; h < 2; ++h) {
+            const int j = j0 + lane + 32 * h;
+            bm[h] = am[h] = cm[h] = 0.0;
             if (j < M) {
-                const double dl = (double)tile[k][jj] * x.zsc[128 + k];   // Q w / d_k
-                const size_t o = (size_t)k * J + j;
-                const double xn = (it > 0 ? xl[o] : 0.0) + dl;
-                if (last) Xl[o] = xn;
-                else xl[o] = xn;
-                sd += dl * dl;
-                sx += xn * xn;
+                bm[h] = t.bm0[j] + xl2 * t.cc[j];
+                if (j == 0) bm[h] = t.bm0[0] + (((m & 1) ? -1.0 : 1.0) - 1.0) * t.ammin + xl2 * t.cc[0];
+                am[h] = t.am[j];
+                cm[h] = t.cm[j];
             }
         }
-        __syncthreads();
+        // d_k r from u = d_k x (the iterate's FP32 part F, or xit times d_k): the
+        // row scales cancel in the radial terms and ride on the vertical
+        // coefficients.  Every load is unconditional, at a column and row clamped
+        // into the arrays (a load under a condition waits for the ones before
+        // it): what lies outside the interior meets zero coefficients (AN(1),
+        // CN(NZ), AM(1), CM(M), the columns past M) or is dropped below.
+        using XT = std::conditional_t<kSrc == 2, double, float>;
+        const int ja = min(j0 + lane, t.J - 1), jb = min(j0 + lane + 32, t.J - 1);
+        const int jh = lane == 31 ? min(j0 + kWideT, t.J - 1) : max(j0 - 1, 0);   // the halo column (lanes 0 and 31)
+        const bool in[2] = {j0 + lane < M, j0 + lane + 32 < M};
+        const XT *it0 = nullptr;
+        if constexpr (kSrc == 1) it0 = Fl;
+        if constexpr (kSrc == 2) it0 = xl;
+        auto scaled = [&](XT f, int k) -> XT {
+            if constexpr (kSrc == 2) return f * c.cd[k].y;
+            else return f;
+        };
+        // the top boundary row, for the warp that holds row NZ
+        const int itop = NZ - 1 - k0;
+        double top[2] = {0.0, 0.0};
+        if (itop >= 0 && itop < 16) {
+            top[0] = Xl[(size_t)NZ * J + ja];
+            top[1] = Xl[(size_t)NZ * J + jb];
+        }
+        float v[2][16];
+        float vmax = 0.0f;
+        XT mid[2] = {};
+        double up[2] = {}, mi[2] = {};   // rows k-1 and k in FP64
+        const int kf = min(k0, NZ - 1);
+        const double *px = Xl + (size_t)kf * J;
+        const XT *pi = it0 + (size_t)kf * t.J;
+        if constexpr (kSrc != 0) {
+            const XT *pu = it0 + (size_t)min(max(k0 - 1, 0), NZ - 1) * t.J;
+            const XT u0 = pu[ja], u1 = pu[jb], m0 = pi[ja], m1 = pi[jb];
+            up[0] = (double)scaled(u0, max(k0 - 1, 0));
+            up[1] = (double)scaled(u1, max(k0 - 1, 0));
+            mid[0] = scaled(m0, k0);
+            mid[1] = scaled(m1, k0);
+            mi[0] = (double)mid[0];
+            mi[1] = (double)mid[1];
+        }
+        const bool edge = j0 + kWideT >= M;   // the tile of column M-1 (or past it)
+#pragma unroll
+        for (int i0 = 0; i0 < 16; i0 += 8) {
+            // this batch's loads: X, the rows below, the halo columns (lane 0: the
+            // one before the tile, lane 31: the one after)
+            double y[2][8];
+            XT dn[2][8], halo[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                y[0][i] = px[ja];
+                y[1][i] = px[jb];
+                if constexpr (kSrc != 0) halo[i] = pi[jh];
+                if (k0 + i0 + i < NZ - 1) {   // uniform; rows NZ and past repeat the last one
+                    px += J;
+                    pi += t.J;
+                }
+                if constexpr (kSrc != 0) {
+                    dn[0][i] = pi[ja];
+                    dn[1][i] = pi[jb];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int k = k0 + i0 + i;
+                const double2 ba = c.ba[k], cd = c.cd[k];
+                // 4 pi G rho with the boundary folds (pot/pot3.f:212-224)
+                const double pg = t.pig4 * cd.y;
+                double r[2] = {pg * y[0][i], pg * y[1][i]};
+                if (i0 + i == itop) {
+                    r[0] = r[0] - t.cnmax * cd.y * top[0];
+                    r[1] = r[1] - t.cnmax * cd.y * top[1];
+                }
+                if (edge) {
+                    const double yM = t.cmmax * cd.y * Xl[(size_t)min(k, NZ - 1) * J + M];
+                    if (j0 + lane == M - 1) r[0] = r[0] - yM;
+                    if (j0 + lane + 32 == M - 1) r[1] = r[1] - yM;
+                }
+                if constexpr (kSrc != 0) {
+                    const XT hv = scaled(halo[i], k);
+                    const XT l0 = __shfl_sync(0xffffffffu, mid[0], lane + 31), l1 = __shfl_sync(0xffffffffu, mid[1], lane + 31);
+                    const XT r0 = __shfl_sync(0xffffffffu, mid[0], lane + 1), r1 = __shfl_sync(0xffffffffu, mid[1], lane + 1);
+                    const XT lf[2] = {lane == 0 ? hv : l0, lane == 0 ? l0 : l1};
+                    const XT rt[2] = {lane == 31 ? r1 : r0, lane == 31 ? hv : r1};
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const XT nx = scaled(dn[h][i], min(k + 1, 127));
+                        const double below = (double)nx;
+                        double ax = (ba.x + bm[h]) * mi[h];
+                        ax += ba.y * up[h];
+                        ax += cd.x * below;
+                        ax += am[h] * (double)lf[h];
+                        ax += cm[h] * (double)rt[h];
+                        r[h] = r[h] - ax;
+                        up[h] = mi[h];
+                        mi[h] = below;
+                        mid[h] = nx;
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float f = in[h] && k < NZ ? (float)r[h] : 0.0f;
+                    v[h][i0 + i] = f;
+                    vmax = fmaxf(vmax, fabsf(f));
+                }
+            }
+        }
+        const float s = pow2_scale(wide_max(c, vmax));
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float a = v[h][8 * g + 2 * i] * s, b = v[h][8 * g + 2 * i + 1] * s;
+                    const __half ah = __float2half_rn(a), bh = __float2half_rn(b);
+                    hi[i] = pack_half2(ah, bh);
+                    lo[i] = pack_half2(__float2half_rn(a - __half2float(ah)), __float2half_rn(b - __half2float(bh)));
+                }
+                const uint32_t o = kmaj_off(lane + 32 * h, k0 + 8 * g, kWideT);
+                *reinterpret_cast<uint4 *>(c.sBh + o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4 *>(c.sBl + o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
+        const bool ok = wide_product(c, false);
+        float *dst = d.W + (size_t)item * d.sw + (size_t)(j0 + 32 * (warp >> 2)) * 128 + 32 * (warp & 3) + lane;
+        const float unscale = 1.0f / (kAScale * s);
+        float o[32];
+        if (ok) tm_ld32(c.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * (warp >> 2), o);
+#pragma unroll
+        for (int u = 0; u < 32; ++u) dst[(size_t)u * 128] = ok ? o[u] * unscale : __int_as_float(0x7fc00000);
     }
-    sd = warp_sum(sd);
-    sx = warp_sum(sx);
-    if ((threadIdx.x & 31) == 0) {
-        red[0][threadIdx.x >> 5] = sd;
-        red[1][threadIdx.x >> 5] = sx;
+    wide_release(c, x.err);
+}
+
+// delta = V w for 64-column tiles of every item, x += delta (FP64).  kSrc: the
+// iterate before (0 none, 1 F / d_k, 2 xit); kDst: where x goes (0 F, 1 xit, 2
+// X's interior).  Each tile's sums of delta^2 and x^2 go to the correction
+// report.
+template <int kSrc, int kDst>
+__global__ void __launch_bounds__(256, 2) k_wide_up(DevTables t, Work w, MixedDev x, WideDev d, int tiles, int it)
+{
+    extern __shared__ __align__(1024) uint8_t sm[];
+    WideCta c;
+    wide_setup(c, sm, t, x);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, M = t.M, NZ = t.NZ;
+    float *stage = reinterpret_cast<float *>(c.sBh);   // [2][128][32], column u of row k at u ^ (k % 32)
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int item = tile / d.nt, j0 = (tile - item * d.nt) * kWideT;
+        // rows j0 + warp + 8 i, values p = 4 lane .. 4 lane + 3
+        const float *src = d.W + (size_t)item * d.sw + (size_t)(j0 + warp) * 128 + 4 * lane;
+        if (tile + (int)gridDim.x < tiles) {   // the next tile: 32 KB of W, 256-byte rows of the iterate
+            const int nt = tile + gridDim.x, ni = nt / d.nt, nj = (nt - ni * d.nt) * kWideT;
+            if (threadIdx.x == 0) l2_prefetch_bulk(d.W + (size_t)ni * d.sw + (size_t)nj * 128, kWideT * 512);
+            if constexpr (kSrc == 1)
+                for (int i = threadIdx.x; i < 2 * NZ; i += 256)
+                    if (nj + 32 * (i & 1) < M) l2_prefetch(d.F + (size_t)ni * d.sx + (size_t)(i >> 1) * t.J + nj + 32 * (i & 1));
+            if constexpr (kSrc == 2)
+                for (int i = threadIdx.x; i < 4 * NZ; i += 256)
+                    if (nj + 16 * (i & 3) < M) l2_prefetch(d.xit + (size_t)ni * d.sx + (size_t)(i >> 2) * t.J + nj + 16 * (i & 3));
+        }
+        float4 v[8];
+        float vmax = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const float4 *>(src + (size_t)i * 8 * 128);
+        // the iterate of this thread's cells of the update
+        const float *Fl = d.F + (size_t)item * d.sx;
+        float f[2][16];
+        const int ja = min(j0 + lane, t.J - 1), jb = min(j0 + lane + 32, t.J - 1);   // loads without conditions
+        if constexpr (kSrc == 1) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float *fr = Fl + (size_t)min(warp + 8 * i, NZ - 1) * t.J;
+                f[0][i] = fr[ja];
+                f[1][i] = fr[jb];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            vmax = fmaxf(vmax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+        const float s = pow2_scale(wide_max(c, vmax));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float a[4] = {v[i].x * s, v[i].y * s, v[i].z * s, v[i].w * s};
+            __half h[4], lo[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                h[u] = __float2half_rn(a[u]);
+                lo[u] = __float2half_rn(a[u] - __half2float(h[u]));
+            }
+            const uint32_t o = kmaj_off(warp + 8 * i, 4 * lane, kWideT);
+            *reinterpret_cast<uint2 *>(c.sBh + o) = make_uint2(pack_half2(h[0], h[1]), pack_half2(h[2], h[3]));
+            *reinterpret_cast<uint2 *>(c.sBl + o) = make_uint2(pack_half2(lo[0], lo[1]), pack_half2(lo[2], lo[3]));
+        }
+        const bool ok = wide_product(c, true);
+        const float unscale = 1.0f / (kAScale * s);
+        {
+            float o[32];
+            if (ok) tm_ld32(c.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * (warp >> 2), o);
+            float *row = stage + (warp >> 2) * 128 * 32 + (32 * (warp & 3) + lane) * 32;
+#pragma unroll
+            for (int u = 0; u < 32; ++u) row[u ^ lane] = ok ? o[u] * unscale : __int_as_float(0x7fc00000);
+        }
+        __syncthreads();
+        double sd = 0.0, sx = 0.0;
+        double *Xl = w.X + (size_t)item * t.K * t.JX, *xl = d.xit + (size_t)item * d.sx;
+        float *Fo = d.F + (size_t)item * d.sx;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int k = warp + 8 * i;
+            if (k >= NZ) break;
+            const double e = c.ek[k];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = j0 + lane + 32 * h;
+                if (j < M) {
+                    const float q = stage[h * 128 * 32 + k * 32 + (lane ^ (k & 31))];
+                    const double dl = (double)q * e;   // Q w / d_k
+                    double xn = dl;
+                    if constexpr (kSrc == 1) xn = (double)f[h][i] * e + dl;
+                    if constexpr (kSrc == 2) xn = xl[(size_t)k * t.J + j] + dl;
+                    if constexpr (kDst == 0) Fo[(size_t)k * t.J + j] = q;
+                    if constexpr (kDst == 1) xl[(size_t)k * t.J + j] = xn;
+                    if constexpr (kDst == 2) Xl[(size_t)k * t.JX + j] = xn;
+                    sd += dl * dl;
+                    sx += xn * xn;
+                }
+            }
+        }
+        sd = warp_sum(sd);
+        sx = warp_sum(sx);
+        double *rd = reinterpret_cast<double *>(c.red) + 8;   // past the maxima
+        if (lane == 0) {
+            rd[warp] = sd;
+            rd[8 + warp] = sx;
+        }
+        __syncthreads();   // also: the staged product has been read
+        if (threadIdx.x == 0) {
+            double a = 0.0, b = 0.0;
+            for (int i = 0; i < 8; ++i) {
+                a += rd[i];
+                b += rd[8 + i];
+            }
+            double *cr = x.corr + (size_t)tile * 16;
+            cr[2 * it] = a;
+            cr[2 * it + 1] = b;
+        }
+    }
+    wide_release(c, x.err);
+}
+
+// n rows of one half of a sweep, from W and the table tab in steps of D rows
+// (D = 1 or -1), in place: f(row value, table value, row index from 0) is the
+// recurrence.  Whole 16-row chunks at constant offsets, loaded one chunk ahead
+// into a second register set; the rest row by row.
+template <int D, class F>
+__device__ __forceinline__ void wide_rows(float *W, const float *tab, int n, F f)
+{
+    constexpr int U = 16, S = D * 128;
+    float ya[U], ta[U], yb[U], tb[U];
+    const float *lw = W, *lt = tab;
+    int i = 0;
+    auto load = [&](float (&y)[U], float (&c)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            y[u] = lw[u * S];
+            c[u] = __ldg(lt + u * S);
+        }
+        lw += U * S;
+        lt += U * S;
+    };
+    auto run = [&](const float (&y)[U], const float (&c)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) W[u * S] = f(y[u], c[u], i + u);
+        W += U * S;
+        i += U;
+    };
+    const int nf = n / U;
+    if (nf > 0) load(ya, ta);
+#pragma unroll 1
+    for (int c = 0; c < nf; c += 2) {
+        if (c + 1 < nf) load(yb, tb);
+        run(ya, ta);
+        if (c + 2 < nf) load(ya, ta);
+        if (c + 1 < nf) run(yb, tb);
+    }
+#pragma unroll 1
+    for (; i < n; ++i, W += S, lt += S) *W = f(*W, __ldg(lt), i);
+}
+
+// (T_r(m) + lam_p) w = W_p for each p of one item (block), with the sweep
+// table's pivot reciprocals and multipliers: rows [0, h) top-down by the first
+// 128 threads, [h, M) bottom-up by the others, meeting at rows h-1 and h --
+// k_mode_mixed's sweeps on CUDA cores, in place.  The item's rows and table
+// slices are prefetched into L2 whole.  With the two halves one after the other
+// and the loads left to the compiler's unrolling 1.18 ms for the 2048 items of
+// four solves of 512x128x512, 0.36 ms now; with row addresses formed from a
+// run-time step (78 instructions a row) it took 1.39.
+__global__ void __launch_bounds__(256) k_wide_sweep(DevTables t, MixedDev x, WideDev d)
+{
+    extern __shared__ float s_tab[];   // AM of rows [0, h), CM of rows [h, M)
+    __shared__ float meet[2][128];
+    // mode-major, modes l and l + N (same m) side by side and the solves innermost:
+    // the blocks in flight share table slices, and their rows stay in L2
+    const int nb = gridDim.x / t.L, q = blockIdx.x / nb, b = blockIdx.x - q * nb;
+    const int l = (q & 1) ? (q >> 1) + t.N : (q >> 1), item = b * t.L + l;
+    const int p = threadIdx.x & 127, M = t.M;
+    const bool low = threadIdx.x >= 128;   // the bottom-up half
+    const int m = l <= t.N ? l : l - t.N;
+    const int NTs = x.ntile, h = 32 * ((M + 63) / 64);
+    if (threadIdx.x == 0) {
+        l2_prefetch_bulk(d.W + (size_t)item * d.sw, (uint32_t)(M * 512));
+        l2_prefetch_bulk(x.sw_piv + (size_t)m * NTs * 128, (uint32_t)(M * 512));
+        l2_prefetch_bulk(x.sw_mul + (size_t)m * NTs * 128, (uint32_t)(M * 512));
+    }
+    for (int j = threadIdx.x; j < M; j += blockDim.x) s_tab[j] = (float)(j < h ? t.am[j] : t.cm[j]);
+    __syncthreads();
+    const bool live = p < t.NZ;
+    float *W = d.W + (size_t)item * d.sw + p;
+    const float *piv = x.sw_piv + (size_t)m * NTs * 128 + p, *mul = x.sw_mul + (size_t)m * NTs * 128 + p;
+    float yp = 0.0f;
+    if (live) {
+        const float *co = s_tab + (low ? M - 1 : 0);
+        if (!low) {
+            wide_rows<1>(W, piv, h, [&](float y, float rr, int i) { return yp = fmaf(-(co[i] * rr), yp, y * rr); });
+        } else {
+            const size_t o = (size_t)(M - 1) * 128;
+            wide_rows<-1>(W + o, piv + o, M - h, [&](float y, float rr, int i) { return yp = fmaf(-(co[-i] * rr), yp, y * rr); });
+        }
+        meet[low][p] = yp;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0, c = 0.0;
-        for (int i = 0; i < 8; ++i) {
-            a += red[0][i];
-            c += red[1][i];
-        }
-        double *cr = x.corr + (size_t)item * 16;
-        cr[2 * it] = a;
-        cr[2 * it + 1] = c;
+    if (!live) return;
+    const float yt = meet[0][p], yu = meet[1][p], et = __ldg(mul + (size_t)(h - 1) * 128), fu = __ldg(mul + (size_t)h * 128);
+    const float xt = (yt + (1.0f - et) * yu) / ((et + fu) - et * fu);
+    const float xu = yu + (1.0f - fu) * xt;
+    // back over this half's rows from the meeting one
+    float xn = low ? xu : xt;
+    auto back = [&](float y, float c, int) { return xn = y + (1.0f - c) * xn; };
+    if (!low) {
+        W[(size_t)(h - 1) * 128] = xn;
+        wide_rows<-1>(W + (ptrdiff_t)(h - 2) * 128, mul + (ptrdiff_t)(h - 2) * 128, h - 1, back);
+    } else {
+        W[(size_t)h * 128] = xn;
+        wide_rows<1>(W + (size_t)(h + 1) * 128, mul + (size_t)(h + 1) * 128, M - h - 1, back);
     }
 }
 
@@ -2360,16 +2623,23 @@ void chy_mixed_bind_tables(chy_plan *p, char *dev_base)
 // chy_mixed_ensure_iterate when such a count is set.
 static size_t al32(size_t n) { return (n + 31) & ~(size_t)31; }   // doubles, 256-byte pieces
 
+// Doubles of one solve's correction sums: 16 a mode, in the wide pipeline 16 a
+// tile of 64 columns.
+static size_t corr_stride(const chy::HostPlan *hp)
+{
+    return (size_t)hp->L * 16 * (mixed_fused(hp) ? 1 : round64(hp->J) / 64);
+}
+
 size_t chy_mixed_work_doubles(const chy_plan *p)
 {
     if (p->precision != CHY_PREC_MIXED) return 0;
     const chy::HostPlan &hp = p->hp;
-    size_t n = al32((size_t)hp.L * 16 * p->max_batch + 8);
+    size_t n = al32(corr_stride(&hp) * p->max_batch + 8);
     if (!mixed_fused(&hp)) {
-        const size_t items = (size_t)hp.L * p->max_batch, Jt = (size_t)(hp.J + 255) / 256 * 256;
-        n += al32(items * hp.K * hp.J);                  // iterate
-        n += 2 * al32(items * Jt * 128 / 2);             // R, O (FP32)
-        n += 2 * al32(items * (Jt / 256) / 2 + 1);       // rmax, wmax
+        const size_t items = (size_t)hp.L * p->max_batch, Jt = (size_t)round64(hp.J);
+        n += al32(items * Jt * 128 / 2);                 // W (FP32)
+        n += al32(items * hp.NZ * hp.J / 2 + 1);         // F (FP32)
+        n += al32(items * hp.NZ * hp.J);                 // FP64 iterate
     }
     return n;
 }
@@ -2380,7 +2650,7 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
     MixedDev &d = p->mx->dev;
     const chy::HostPlan &hp = p->hp;
     d.sxb = (size_t)hp.L * hp.K * p->t.JX;
-    d.scorr = (size_t)hp.L * 16;
+    d.scorr = corr_stride(&hp);
     d.xbuf = nullptr;
     d.corr = base;
     d.err = reinterpret_cast<int *>(d.corr + d.scorr * p->max_batch);
@@ -2389,20 +2659,15 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
         WideDev &wd = p->mx->wide;
         p->mx->is_wide = true;
         const size_t items = (size_t)hp.L * p->max_batch;
-        wd.Jt = (hp.J + 255) / 256 * 256;
-        wd.nt = wd.Jt / 256;
-        double *q = base + al32((size_t)hp.L * 16 * p->max_batch + 8);
+        wd.nt = round64(hp.J) / 64;
+        wd.sw = (size_t)round64(hp.J) * 128;
+        wd.sx = (size_t)hp.NZ * hp.J;
+        double *q = base + al32(d.scorr * p->max_batch + 8);
+        wd.W = reinterpret_cast<float *>(q);
+        q += al32(items * wd.sw / 2);
+        wd.F = reinterpret_cast<float *>(q);
+        q += al32(items * wd.sx / 2 + 1);
         wd.xit = q;
-        wd.sxit = (size_t)hp.K * hp.J;
-        q += al32(items * hp.K * hp.J);
-        wd.sro = (size_t)wd.Jt * 128;
-        wd.R = reinterpret_cast<float *>(q);
-        q += al32(items * wd.sro / 2);
-        wd.O = reinterpret_cast<float *>(q);
-        q += al32(items * wd.sro / 2);
-        wd.rmax = reinterpret_cast<unsigned *>(q);
-        q += al32(items * wd.nt / 2 + 1);
-        wd.wmax = reinterpret_cast<unsigned *>(q);
     }
     if (p->precision == CHY_PREC_MIXED) {
         cudaMallocHost(&p->mx->h_corr, sizeof(double) * d.scorr * p->max_batch);
@@ -2439,28 +2704,33 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
     }
 }
 
+template <class Kernel, class... Args>
+static int wide_launch(Kernel kern, const chy_plan *p, int tiles, cudaStream_t s, Args... args)
+{
+    if (ensure_smem((const void *)kern, WideSmem::bytes) != cudaSuccess) return CHY_ERR_CUDA;
+    kern<<<std::min(tiles, 2 * p->num_sms), 256, WideSmem::bytes, s>>>(p->t, p->w, p->mx->dev, p->mx->wide, tiles, args...);
+    return cudaGetLastError() == cudaSuccess ? CHY_OK : CHY_ERR_CUDA;
+}
+
 static int wide_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
 {
-    const MixedDev &x = p->mx->dev;
     const WideDev &d = p->mx->wide;
     const chy::DevTables &t = p->t;
-    const int nit = std::min(1 + p->refine, 8), items = nb * t.L;
-    const size_t gsm = (size_t)kAImg + (size_t)kWideN * 512 + 64;
-    if (ensure_smem((const void *)k_wide_gemm, gsm) != cudaSuccess) return CHY_ERR_CUDA;
+    const int nit = std::min(1 + p->refine, 8), items = nb * t.L, tiles = items * d.nt;
     for (int it = 0; it < nit; ++it) {
-        const size_t mb = (size_t)items * d.nt * sizeof(unsigned);
-        if (cudaMemsetAsync(d.rmax, 0, mb, s) != cudaSuccess || cudaMemsetAsync(d.wmax, 0, mb, s) != cudaSuccess)
-            return CHY_ERR_CUDA;
-        const dim3 rg(d.Jt / 32, items), gg(d.nt, items);
-        if (it == 0) k_wide_resid<true><<<rg, 256, 0, s>>>(t, p->w, x, d, nb);
-        else k_wide_resid<false><<<rg, 256, 0, s>>>(t, p->w, x, d, nb);
-        k_wide_gemm<<<gg, 256, gsm, s>>>(x.aimg, d.R, d.O, d.rmax, d, 0, x.err);
-        k_wide_sweep<<<items, 128, 2 * t.M * sizeof(float), s>>>(t, x, d);
-        k_wide_gemm<<<gg, 256, gsm, s>>>(x.aimg, d.R, d.O, d.wmax, d, 1, x.err);
-        k_wide_update<<<items, 256, 0, s>>>(t, p->w, x, d, it, it == nit - 1 ? 1 : 0);
+        const bool last = it == nit - 1;
+        int st = it == 0   ? wide_launch(k_wide_down<0>, p, tiles, s)
+                 : it == 1 ? wide_launch(k_wide_down<1>, p, tiles, s)
+                           : wide_launch(k_wide_down<2>, p, tiles, s);
+        if (st != CHY_OK) return st;
+        k_wide_sweep<<<items, 256, t.M * sizeof(float), s>>>(t, p->mx->dev, d);
         if (cudaGetLastError() != cudaSuccess) return CHY_ERR_CUDA;
+        st = it == 0   ? (last ? wide_launch(k_wide_up<0, 2>, p, tiles, s, it) : wide_launch(k_wide_up<0, 0>, p, tiles, s, it))
+             : it == 1 ? (last ? wide_launch(k_wide_up<1, 2>, p, tiles, s, it) : wide_launch(k_wide_up<1, 1>, p, tiles, s, it))
+                       : (last ? wide_launch(k_wide_up<2, 2>, p, tiles, s, it) : wide_launch(k_wide_up<2, 1>, p, tiles, s, it));
+        if (st != CHY_OK) return st;
     }
-    *launches = 5 * nit;
+    *launches = 3 * nit;
     return CHY_OK;
 }
 
@@ -2593,9 +2863,10 @@ void chy_mixed_fill_diag(const chy_plan *p, int slot, chy_diag *d)
     d->iterations = nit;
     // k_mode_pair leaves one sum per radial half: [0, 4) and [8, 12)
     const bool halves = p->mx->paired;
+    const int rows = (int)(p->mx->dev.scorr / 16);   // modes, in the wide pipeline their tiles
     for (int it = 0; it < nit && it < 8; ++it) {
         double sd = 0.0, sx = 0.0;
-        for (int l = 0; l < p->hp.L; ++l) {
+        for (int l = 0; l < rows; ++l) {
             sd += c[(size_t)l * 16 + 2 * it];
             sx += c[(size_t)l * 16 + 2 * it + 1];
             if (halves) {
