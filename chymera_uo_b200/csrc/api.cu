@@ -13,6 +13,7 @@
 
 #include "chy_pot3.h"
 #include "chy_pot3_testing.h"
+#include "pdl.h"
 #include "planimpl.h"
 
 using namespace chy;
@@ -617,10 +618,12 @@ long long chy_plan_launch_count(const chy_plan *p) { return p ? p->launches : 0;
 // Event sets kept before older ones are folded in (with a host wait).
 static constexpr size_t kMaxEventSets = 4096;
 
-// One launch sequence over nb solves whose caller buffers are in bp.
-static int run_batch(chy_plan *p, const BatchPtrs &bp, int nb, cudaStream_t s)
+// One launch sequence over nb solves whose caller buffers are in bp.  alone: no
+// other launch sequence of this library is meant to run beside it.
+static int run_batch(chy_plan *p, const BatchPtrs &bp, int nb, cudaStream_t s, bool alone)
 {
     const DevTables &t = p->t;
+    p->w.pdl = alone && nb * p->nvol <= kPdlCells;
     const bool prof = p->profile;
     cudaEvent_t *evs = nullptr;
     if (prof) {
@@ -732,7 +735,7 @@ extern "C" int chy_solve_batch(chy_plan *p, int n, const double *const *rho, dou
             const int nb = std::min(std::min(n - first, p->max_batch), kMaxBatchPtrs);
             BatchPtrs bp{};
             for (int i = 0; i < nb; i++) { bp.rho[i] = rho[first + i]; bp.phi[i] = phi[first + i]; }
-            int st = run_batch(p, bp, nb, s);
+            int st = run_batch(p, bp, nb, s, true);
             if (st != CHY_OK) return st;
             st = fetch_diag(p, diag, nb, first, s);
             if (st != CHY_OK) return st;
@@ -783,7 +786,7 @@ extern "C" int chy_solve_batch(chy_plan *p, int n, const double *const *rho, dou
         // caller's values: the device buffer starts from the host array
         if (p->coef_host)
             CHY_CUDA(cudaMemcpyAsync(p->coef_dev, p->coef_host, p->coef_bytes, cudaMemcpyHostToDevice, s));
-        st = run_batch(p, bp, nb, s);
+        st = run_batch(p, bp, nb, s, true);
         if (st != CHY_OK) return st;
         if (p->coef_host)
             CHY_CUDA(cudaMemcpyAsync(p->coef_host, p->coef_dev, p->coef_bytes, cudaMemcpyDeviceToHost, s));
@@ -904,7 +907,7 @@ extern "C" int chy_solve_multi(int n, chy_plan *const *plans, const double *cons
                 bp.rho[i] = rho[idx[first + i]];
                 bp.phi[i] = phi[idx[first + i]];
             }
-            st = run_batch(p, bp, nb, gs);
+            st = run_batch(p, bp, nb, gs, S == 1);
             if (st != CHY_OK) return st;
             first += nb;
         }
@@ -1065,7 +1068,7 @@ size_t chy_internal_drop_blk_table(chy_plan *p)
     return bytes;
 }
 
-int chy_internal_run_batch(chy_plan *p, const BatchPtrs &bp, int nb, cudaStream_t s) { return run_batch(p, bp, nb, s); }
+int chy_internal_run_batch(chy_plan *p, const BatchPtrs &bp, int nb, cudaStream_t s) { return run_batch(p, bp, nb, s, false); }
 
 const double *chy_internal_mapped_view(const double *host)
 {
@@ -1208,6 +1211,7 @@ extern "C" int chy_solve_static(chy_plan *p, const double *rho, double *phi, voi
     w.phac = q; q += al(pw.sphac);
     w.diag = q;
     w.coef = nullptr;   // /COEFS/ output only through chy_solve
+    w.pdl = p->nvol <= kPdlCells;
     cudaStream_t s = (cudaStream_t)stream;
     // every call starts from zeroed work space, as the plan's own allocation does
     CHY_CUDA(cudaMemsetAsync(base, 0, need * sizeof(double), s));

@@ -108,6 +108,7 @@ struct Work {
     size_t sX, sW, smom, ssub, sscan, sphac, sdiag;   // per-solve strides (elements)
     double *coef;                                    // optional /COEFS/ output (solve 0 only)
     double *bvec, *bscr;                             // BLKTRI-order path (k_blktri.cu)
+    bool pdl;                                        // overlap launches (pdl.h)
 };
 
 // ExternalPot (pot/ExternalPot.f:1-80): the star potential added after POT3.

@@ -17,6 +17,7 @@
 // Compiled with --fmad=false: each product and sum rounds separately, in a
 // fixed order.
 #include "devplan.h"
+#include "pdl.h"
 
 namespace chy {
 
@@ -39,6 +40,7 @@ __global__ void __launch_bounds__(kSubThreads) k_bdy_sub(DevTables t, Work w, in
     const int sc = blockIdx.x;
     const int s0 = t.sub_start[sc], s1 = t.sub_start[sc + 1], ns = s1 - s0;
 
+    pdl_go();
     // per ring, geometry from the plan (TERM(I) of pot/boundary.f:385-502,
     // r^-(2l+1) of :587, DV of :516): asynchronous copies, under way while the
     // moments are gathered into registers
@@ -54,6 +56,7 @@ __global__ void __launch_bounds__(kSubThreads) k_bdy_sub(DevTables t, Work w, in
                          "l"(row + i)
                          : "memory");
     }
+    pdl_wait();
     const int b0 = blockIdx.z * kSubBatch, b1 = min(nb, b0 + kSubBatch);
     for (int b = b0; b < b1; b += spp) {
         const int nsl = min(spp, b1 - b);
@@ -160,6 +163,8 @@ constexpr int kScanCols = 16, kScanRuns = 64, kScanRegs = 16;
 __global__ void __launch_bounds__(kScanCols *kScanRuns) k_bdy_scan(DevTables t, Work w)
 {
     __shared__ double run_tot[kScanRuns][kScanCols];
+    pdl_go();
+    pdl_wait();
     const int lane = threadIdx.x % kScanCols, seg = threadIdx.x / kScanCols, b = blockIdx.z;
     const int cc = blockIdx.x * kScanCols + lane, ld = 2 * t.ncol;
     const bool live = cc < ld, out = cc >= t.ncol;
@@ -235,11 +240,9 @@ cudaError_t launch_bdy_sums(const DevTables &t, const Work &w, int nb, cudaStrea
     const size_t sm = (size_t)kSubChunk * (t.srow + 21 * spp) * sizeof(double);
     cudaError_t e = ensure_smem((const void *)k_bdy_sub, sm);
     if (e != cudaSuccess) return e;
-    k_bdy_sub<<<dim3(t.nsub, 1, (nb + kSubBatch - 1) / kSubBatch), threads, sm, s>>>(t, w, nb, spp);
-    e = cudaGetLastError();
+    e = launch_pdl(w.pdl, k_bdy_sub, dim3(t.nsub, 1, (nb + kSubBatch - 1) / kSubBatch), dim3(threads), sm, s, t, w, nb, spp);
     if (e != cudaSuccess) return e;
-    k_bdy_scan<<<dim3((2 * t.ncol + kScanCols - 1) / kScanCols, 1, nb), kScanCols * kScanRuns, 0, s>>>(t, w);
-    return cudaGetLastError();
+    return launch_pdl(w.pdl, k_bdy_scan, dim3((2 * t.ncol + kScanCols - 1) / kScanCols, 1, nb), dim3(kScanCols * kScanRuns), 0, s, t, w);
 }
 
 }  // namespace chy

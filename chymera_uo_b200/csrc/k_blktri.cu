@@ -21,6 +21,7 @@
 // every product, sum and quotient rounds as the reference's, so the modes equal
 // the reference's BLKTRI output bit for bit.
 #include "devplan.h"
+#include "pdl.h"
 
 #include <type_traits>
 
@@ -48,6 +49,8 @@ __global__ void __launch_bounds__(256) k_blk_gather(DevTables t, Work w, int nb)
     const int M = t.M, L = t.L;
     const BlkDev &d = t.blk;
     double *out = w.bvec + ((size_t)g * d.nvec + k) * (size_t)M * kBlkLanes;
+    pdl_go();
+    pdl_wait();
     const int j0 = blockIdx.z * kBlkLanes;
     for (int r = ty; r < kBlkLanes; r += 8) {
         const int item = g * kBlkLanes + r, b = item / L, l = item % L, j = j0 + tx;
@@ -70,6 +73,8 @@ __global__ void __launch_bounds__(256) k_blk_scatter(DevTables t, Work w, int nb
     const int M = t.M, L = t.L;
     const BlkDev &d = t.blk;
     const double *in = w.bvec + ((size_t)g * d.nvec + k) * (size_t)M * kBlkLanes;
+    pdl_go();
+    pdl_wait();
     const int j0 = blockIdx.z * kBlkLanes;
     for (int jj = ty; jj < kBlkLanes; jj += 8) {
         const int j = j0 + jj;
@@ -658,6 +663,8 @@ __global__ void __launch_bounds__(128, 1) k_blk_solve_tab(DevTables t, Work w, i
     }
     __syncthreads();
     if constexpr (TM) bw.tm = tm_base + ((uint32_t)(warp * 32) << 16);
+    pdl_go();
+    pdl_wait();
     const size_t rstride = (size_t)d.ntab * 3 * col;
     const int worker = rank + ctas * warp, workers = ctas * nw;
     for (int g = slot; g < ngroups; g += slots) {
@@ -812,12 +819,14 @@ static cudaError_t blk_solve_tab(const DevTables &t, const Work &w, int ngroups,
     cfg.blockDim = dim3(nw * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = ctas;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = ctas > 1 ? 1 : 0;
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = w.pdl ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, k_blk_solve_tab<TM>, t, w, ngroups, ctas);
 }
 
@@ -830,8 +839,7 @@ cudaError_t launch_solve_blk(const DevTables &t, const Work &w, int nb, int num_
     // the scratch (16 per SM, no more than 16 per group)
     const int cap = ctas_per_sm * num_sms, ctas = ngroups < cap ? ngroups : cap;
     const int rtiles = (t.M + kBlkLanes - 1) / kBlkLanes;
-    k_blk_gather<<<dim3(ngroups, t.NZ, rtiles), 256, 0, s>>>(t, w, nb);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_pdl(w.pdl, k_blk_gather, dim3(ngroups, t.NZ, rtiles), dim3(256), 0, s, t, w, nb);
     if (e != cudaSuccess) return e;
     if (t.blk.tab)
         e = blk_tab_tm(t.M) ? blk_solve_tab<true>(t, w, ngroups, num_sms, nw, s)
@@ -840,9 +848,8 @@ cudaError_t launch_solve_blk(const DevTables &t, const Work &w, int nb, int num_
     else if (nw == 8) e = blk_launch<8>(t, w, ngroups, ctas, s);
     else e = blk_launch<16>(t, w, ngroups, ctas, s);
     if (e != cudaSuccess) return e;
-    k_blk_scatter<<<dim3(ngroups, t.NZ, rtiles), 256, 0, s>>>(t, w, nb);
     if (launches) *launches = 3;
-    return cudaGetLastError();
+    return launch_pdl(w.pdl, k_blk_scatter, dim3(ngroups, t.NZ, rtiles), dim3(256), 0, s, t, w, nb);
 }
 
 }  // namespace chy

@@ -19,6 +19,7 @@
 // permutation and REALTR recurrence values are the recorded tables, staged in
 // shared memory.
 #include "devplan.h"
+#include "pdl.h"
 
 #include <cstring>
 #include <type_traits>
@@ -356,12 +357,16 @@ __global__ void __launch_bounds__(256) k_forward(DevTables t, BatchPtrs bp, Work
     // solve's RHO, counted on tbar (after the tables)
     uint64_t *tbar = reinterpret_cast<uint64_t *>(smem_raw + (size_t)T::ROWS * T::RS * 8 + (size_t)20 * (L / 4) * 8 +
                                                   fft_table_bytes<L>());
+    pdl_go();
     if (vec16 == 2) {
         if (threadIdx.x == 0) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sm32(tbar)));
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncthreads();
+    }
+    pdl_wait();
+    if (vec16 == 2) {
         if (threadIdx.x == 0) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sm32(tbar)),
                          "r"((uint32_t)(L * T::RS * 8) + fft_bulk_bytes(t.fwd) + 20u * (L / 4) * 8u));
@@ -546,12 +551,14 @@ __global__ void __launch_bounds__(256) k_bdy_synth(DevTables t, Work w)
     const double *scan = w.scan + (size_t)b * w.sscan;
     // one azimuth l per thread: its 21 basis values serve the block's kPts
     // boundary points; the first azimuth's are on their way from the start
+    pdl_go();
     double f[21];
     int l = threadIdx.x;
     if (l < L) {
 #pragma unroll
         for (int p = 0; p < 21; ++p) f[p] = __ldg(t.fbasis + (size_t)p * L + l);
     }
+    pdl_wait();
     // TRMTOT: all of a thread's loads in flight together
     constexpr int NT = (kPts * 132 + 255) / 256;
     double vi[NT], vo[NT], bi[NT], bo[NT];
@@ -767,12 +774,16 @@ __global__ void __launch_bounds__(256) k_inverse(DevTables t, BatchPtrs bp, Work
     // TC columns x one K x up to 256 modes: modes 0..N-1 into rows 0..N-1 and
     // modes N..2N-1 into rows IM0..IM0+N-1; mode N then moves to row N and rows
     // IM0 and IM0+N become B1(1) = B1(N+1) = 0
+    pdl_go();
     if (xmode == 2) {
         if (threadIdx.x == 0) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sm32(tbar)));
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncthreads();
+    }
+    pdl_wait();
+    if (xmode == 2) {
         if (threadIdx.x == 0) {
             constexpr int B = n < 256 ? n : 256;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sm32(tbar)),
@@ -914,6 +925,8 @@ __global__ void __launch_bounds__(128) k_star_rim(DevTables t, BatchPtrs bp, Wor
 {
     const int l = blockIdx.x, b = blockIdx.y, J2 = t.J + 2, K2 = t.K + 2;
     double *phi = bp.phi[b];
+    pdl_go();
+    pdl_wait();
     double ix, iy;
     star_pos(x, w, b, &ix, &iy);
     for (int j = threadIdx.x; j <= J2; j += blockDim.x) {
@@ -941,6 +954,8 @@ __global__ void __launch_bounds__(32 * kMomWarps) k_star_moment(DevTables t, Bat
     const double *rho = bp.rho[b] + (size_t)J2 * K2 * l;
     const int j0 = x.jmin - 1;   // 0-based J = JMIN-1 .. JMAX
     const double c = t.cosm[l], s = t.sinm[l];
+    pdl_go();
+    pdl_wait();
     double sx = 0.0, sy = 0.0;
     constexpr int U = 4;
     for (int jb = j0 + lane; jb <= t.J; jb += 32 * U) {
@@ -996,6 +1011,8 @@ __global__ void __launch_bounds__(32 * kMomWarps) k_star_moment(DevTables t, Bat
 __global__ void k_star_shift(DevTables t, Work w, StarDev x)
 {
     const int b = blockIdx.x;
+    pdl_go();
+    pdl_wait();
     double *d = w.diag + (size_t)b * w.sdiag;
     double sx = 0.0, sy = 0.0;
     for (int l = threadIdx.x; l < t.L; l += 32) {
@@ -1030,6 +1047,8 @@ __global__ void __launch_bounds__(128) k_star_fill(DevTables t, Work w, StarDev 
 __global__ void __launch_bounds__(32) k_diag(DevTables t, Work w)
 {
     const int b = blockIdx.x, lane = threadIdx.x;
+    pdl_go();
+    pdl_wait();
     const double *phac = w.phac + (size_t)b * w.sphac;
     double err = 0.0;
     int klocat = 0;
@@ -1102,8 +1121,7 @@ static cudaError_t forward_l(const DevTables &t, const BatchPtrs &bp, const Work
     }
     // 256 threads: the table copies, the moment halves and the compile-time
     // trip counts of k_forward assume eight warps
-    k_forward<L><<<dim3((t.M + T::TC - 1) / T::TC, t.NZ, nb), 256, sm, s>>>(t, bp, w, vec16, maps);
-    return cudaGetLastError();
+    return launch_pdl(w.pdl, k_forward<L>, dim3((t.M + T::TC - 1) / T::TC, t.NZ, nb), dim3(256), sm, s, t, bp, w, vec16, maps);
 }
 
 template <int L>
@@ -1132,16 +1150,15 @@ static cudaError_t inverse_l(const DevTables &t, const BatchPtrs &bp, const Work
     }
     // 256 threads: the table copies and the compile-time trip counts of
     // k_inverse assume eight warps
-    k_inverse<L><<<dim3((t.J + T::TC - 1) / T::TC, t.K, nb), 256, sm, s>>>(t, bp, w, x, xmode, xmap);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_pdl(w.pdl, k_inverse<L>, dim3((t.J + T::TC - 1) / T::TC, t.K, nb), dim3(256), sm, s, t, bp, w, x, xmode, xmap);
+    if (e != cudaSuccess) return e;
     *launches = 2;
     if (x.on) {
-        k_star_rim<<<dim3(L, nb), 128, 0, s>>>(t, bp, w, x);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        e = launch_pdl(false, k_star_rim, dim3(L, nb), dim3(128), 0, s, t, bp, w, x);
+        if (e != cudaSuccess) return e;
         *launches = 3;
     }
-    k_diag<<<nb, 32, 0, s>>>(t, w);
-    return cudaGetLastError();
+    return launch_pdl(w.pdl, k_diag, dim3(nb), dim3(32), 0, s, t, w);
 }
 
 #define CHY_DISPATCH_L(FN, ...)                     \
@@ -1162,8 +1179,7 @@ cudaError_t launch_forward(const DevTables &t, const BatchPtrs &bp, const Work &
 
 cudaError_t launch_bdy_synth(const DevTables &t, const Work &w, int nb, cudaStream_t s)
 {
-    k_bdy_synth<<<dim3((t.njk + 7) / 8, 1, nb), 256, 0, s>>>(t, w);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_pdl(w.pdl, k_bdy_synth, dim3((t.njk + 7) / 8, 1, nb), dim3(256), 0, s, t, w);
     if (e != cudaSuccess || w.coef == nullptr) return e;
     k_coef<<<dim3((t.J + 31) / 32, t.K, 1), dim3(32, 8), 0, s>>>(t, w);
     return cudaGetLastError();
@@ -1178,11 +1194,9 @@ cudaError_t launch_inverse(const DevTables &t, const BatchPtrs &bp, const Work &
 cudaError_t launch_star_shift(const DevTables &t, const BatchPtrs &bp, const Work &w, const StarDev &x, int nb,
                               cudaStream_t s)
 {
-    k_star_moment<<<dim3(t.L, nb), 32 * kMomWarps, 0, s>>>(t, bp, w, x);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_pdl(false, k_star_moment, dim3(t.L, nb), dim3(32 * kMomWarps), 0, s, t, bp, w, x);
     if (e != cudaSuccess) return e;
-    k_star_shift<<<nb, 32, 0, s>>>(t, w, x);
-    return cudaGetLastError();
+    return launch_pdl(false, k_star_shift, dim3(nb), dim3(32), 0, s, t, w, x);
 }
 
 cudaError_t launch_star_fill(const DevTables &t, const Work &w, const StarDev &x, int slot, double *out,

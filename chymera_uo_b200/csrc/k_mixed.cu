@@ -36,6 +36,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "pdl.h"
 #include "planimpl.h"
 
 using namespace chy;
@@ -501,6 +502,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_mixed(DevTables t, Work w, Mixe
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_cv + 1);
     int *s_flag = reinterpret_cast<int *>(tmem_slot + 1);
 
+    pdl_go();
     // ---- setup: tensor memory (all 512 columns), barriers, m-independent tables
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
@@ -592,6 +594,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_mixed(DevTables t, Work w, Mixe
         }
     };
 
+    pdl_wait();
     for (long long item = blockIdx.x; item < items && !failed; item += gridDim.x) {
         fail_item = item;
         // mode-major order, modes l and l + N (same m) side by side and the
@@ -1370,6 +1373,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_pair(DevTables t, Work w, Mixed
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + PairSmem::misc);
     int *s_flag = reinterpret_cast<int *>(sm + PairSmem::misc + 8) ;   // [2]
 
+    pdl_go();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -1391,6 +1395,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_pair(DevTables t, Work w, Mixed
     __syncthreads();
     // the peer's barriers are initialised before anything is sent to them
     cluster_sync_all();
+    pdl_wait();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
@@ -2086,7 +2091,9 @@ __global__ void __launch_bounds__(256, 2) k_wide_down(DevTables t, Work w, Mixed
 {
     extern __shared__ __align__(1024) uint8_t sm[];
     WideCta c;
+    pdl_go();
     wide_setup(c, sm, t, x);
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, M = t.M, NZ = t.NZ, J = t.JX, k0 = 16 * warp;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int item = tile / d.nt, j0 = (tile - item * d.nt) * kWideT;
@@ -2262,7 +2269,9 @@ __global__ void __launch_bounds__(256, 2) k_wide_up(DevTables t, Work w, MixedDe
 {
     extern __shared__ __align__(1024) uint8_t sm[];
     WideCta c;
+    pdl_go();
     wide_setup(c, sm, t, x);
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, M = t.M, NZ = t.NZ;
     float *stage = reinterpret_cast<float *>(c.sBh);   // [2][128][32], column u of row k at u ^ (k % 32)
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -2428,13 +2437,15 @@ __global__ void __launch_bounds__(256) k_wide_sweep(DevTables t, MixedDev x, Wid
     const bool low = threadIdx.x >= 128;   // the bottom-up half
     const int m = l <= t.N ? l : l - t.N;
     const int NTs = x.ntile, h = 32 * ((M + 63) / 64);
+    pdl_go();
     if (threadIdx.x == 0) {
-        l2_prefetch_bulk(d.W + (size_t)item * d.sw, (uint32_t)(M * 512));
         l2_prefetch_bulk(x.sw_piv + (size_t)m * NTs * 128, (uint32_t)(M * 512));
         l2_prefetch_bulk(x.sw_mul + (size_t)m * NTs * 128, (uint32_t)(M * 512));
     }
     for (int j = threadIdx.x; j < M; j += blockDim.x) s_tab[j] = (float)(j < h ? t.am[j] : t.cm[j]);
     __syncthreads();
+    pdl_wait();
+    if (threadIdx.x == 0) l2_prefetch_bulk(d.W + (size_t)item * d.sw, (uint32_t)(M * 512));
     const bool live = p < t.NZ;
     float *W = d.W + (size_t)item * d.sw + p;
     const float *piv = x.sw_piv + (size_t)m * NTs * 128 + p, *mul = x.sw_mul + (size_t)m * NTs * 128 + p;
@@ -2708,8 +2719,10 @@ template <class Kernel, class... Args>
 static int wide_launch(Kernel kern, const chy_plan *p, int tiles, cudaStream_t s, Args... args)
 {
     if (ensure_smem((const void *)kern, WideSmem::bytes) != cudaSuccess) return CHY_ERR_CUDA;
-    kern<<<std::min(tiles, 2 * p->num_sms), 256, WideSmem::bytes, s>>>(p->t, p->w, p->mx->dev, p->mx->wide, tiles, args...);
-    return cudaGetLastError() == cudaSuccess ? CHY_OK : CHY_ERR_CUDA;
+    return launch_pdl(p->w.pdl, kern, dim3(std::min(tiles, 2 * p->num_sms)), dim3(256), WideSmem::bytes, s, p->t, p->w, p->mx->dev,
+                      p->mx->wide, tiles, args...) == cudaSuccess
+               ? CHY_OK
+               : CHY_ERR_CUDA;
 }
 
 static int wide_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
@@ -2723,8 +2736,7 @@ static int wide_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
                  : it == 1 ? wide_launch(k_wide_down<1>, p, tiles, s)
                            : wide_launch(k_wide_down<2>, p, tiles, s);
         if (st != CHY_OK) return st;
-        k_wide_sweep<<<items, 256, t.M * sizeof(float), s>>>(t, p->mx->dev, d);
-        if (cudaGetLastError() != cudaSuccess) return CHY_ERR_CUDA;
+        if (launch_pdl(p->w.pdl, k_wide_sweep, dim3(items), dim3(256), t.M * sizeof(float), s, t, p->mx->dev, d) != cudaSuccess) return CHY_ERR_CUDA;
         st = it == 0   ? (last ? wide_launch(k_wide_up<0, 2>, p, tiles, s, it) : wide_launch(k_wide_up<0, 0>, p, tiles, s, it))
              : it == 1 ? (last ? wide_launch(k_wide_up<1, 2>, p, tiles, s, it) : wide_launch(k_wide_up<1, 1>, p, tiles, s, it))
                        : (last ? wide_launch(k_wide_up<2, 2>, p, tiles, s, it) : wide_launch(k_wide_up<2, 1>, p, tiles, s, it));
@@ -2780,17 +2792,19 @@ int chy_mixed_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
             pairs = std::min<long long>(pairs, ms.pair_clusters);
             pairs = std::min<long long>(pairs, std::max(1, cap / 2));
             cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute at[1];
+            cudaLaunchAttribute at[2] = {};
             at[0].id = cudaLaunchAttributeClusterDimension;
             at[0].val.clusterDim.x = 2;
             at[0].val.clusterDim.y = 1;
             at[0].val.clusterDim.z = 1;
+            at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.gridDim = dim3(2 * (unsigned)pairs, 1, 1);
             cfg.blockDim = dim3(256, 1, 1);
             cfg.dynamicSmemBytes = PairSmem::bytes;
             cfg.stream = s;
             cfg.attrs = at;
-            cfg.numAttrs = 1;
+            cfg.numAttrs = p->w.pdl ? 2 : 1;
             if (cudaLaunchKernelEx(&cfg, k_mode_pair, p->t, p->w, d, nb, p->mx->tm_pl, p->mx->tm_ps, p->mx->tm_psl) != cudaSuccess)
                 return CHY_ERR_CUDA;
             ms.paired = true;
@@ -2803,9 +2817,9 @@ int chy_mixed_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
     cudaError_t e = ensure_smem(kern, sm);
     if (e != cudaSuccess) return CHY_ERR_CUDA;
     const int grid = (int)(items < cap ? items : cap);
-    if (d.nit <= 2) k_mode_mixed<true><<<grid, 256, sm, s>>>(p->t, p->w, d, nb, p->mx->tm_x, p->mx->tm_xs);
-    else k_mode_mixed<false><<<grid, 256, sm, s>>>(p->t, p->w, d, nb, p->mx->tm_x, p->mx->tm_xs);
-    if (cudaGetLastError() != cudaSuccess) return CHY_ERR_CUDA;
+    e = launch_pdl(p->w.pdl, d.nit <= 2 ? k_mode_mixed<true> : k_mode_mixed<false>, dim3(grid), dim3(256), sm, s, p->t, p->w, d, nb, p->mx->tm_x,
+                   p->mx->tm_xs);
+    if (e != cudaSuccess) return CHY_ERR_CUDA;
     *launches = 1;
     return CHY_OK;
 }

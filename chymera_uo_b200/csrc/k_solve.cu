@@ -29,6 +29,7 @@
 // these (0.665 / 0.659 ms against 0.661 / 0.642); 64-bit item divisions in
 // every warp cost 0.02-0.05 ms.
 #include "devplan.h"
+#include "pdl.h"
 
 namespace chy {
 
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd_f64(DevTables t, Work w, 
     extern __shared__ __align__(16) double smem[];   // [3][KP][LDY]
     const int NZ = t.NZ, M = t.M, J = t.J, K = t.K, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wp = warp % Z::NWP, wj = warp / Z::NWP;
+    pdl_go();
     double u[Z::KS];
 #pragma unroll
     for (int s = 0; s < Z::KS; ++s) {
@@ -93,6 +95,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd_f64(DevTables t, Work w, 
     // rows k >= K and columns no copy reaches start as zeros
     for (int i = tid; i < 3 * Z::kFwdBuf; i += kZThreads) smem[i] = 0.0;
     __syncthreads();
+    pdl_wait();
     const int njt = (M + Z::JT - 1) / Z::JT;
     const int items = nb * t.L * njt;   // item = (solve * L + mode) * njt + tile
     const bool even = (J & 1) == 0;
@@ -198,8 +201,10 @@ __global__ void __launch_bounds__(128) k_thomas_f64(DevTables t, Work w)
     const int M = t.M, K = KC ? KC : t.K, p = threadIdx.x % K, b = blockIdx.y;
     const int l = blockIdx.x * (blockDim.x / K) + threadIdx.x / K;
     extern __shared__ double am[];
+    pdl_go();
     for (int j = threadIdx.x; j < M; j += blockDim.x) am[j] = t.am[j];
     __syncthreads();
+    pdl_wait();
     if (p >= t.NZ || l >= t.L) return;
     double *Wp = w.W + (size_t)b * w.sW + (size_t)l * t.J * K + p;
     const size_t tab = (size_t)mode_m(l, t.N) * M * K + p;
@@ -285,6 +290,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zinv_f64(DevTables t, Work w, 
     const int NZ = t.NZ, M = t.M, J = t.J, K = t.K, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wk = warp % Z::NWP, wj = warp / Z::NWP;
     const int k = wk * 8 + lane / 4;
+    pdl_go();
     double va[Z::KS];
 #pragma unroll
     for (int s = 0; s < Z::KS; ++s) {
@@ -294,6 +300,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zinv_f64(DevTables t, Work w, 
     // columns p >= K of narrow grids and rows no copy reaches start as zeros
     for (int i = tid; i < 3 * Z::kInvBuf; i += kZThreads) smem[i] = 0.0;
     __syncthreads();
+    pdl_wait();
     const int njt = (M + Z::JT - 1) / Z::JT;
     const int items = nb * t.L * njt;
     const int h = K / 2, hs = __ffs(h) - 1;   // KMAX is a power of two
@@ -364,13 +371,12 @@ static cudaError_t solve_fp64(const DevTables &t, const Work &w, int nb, int num
     if (e == cudaSuccess) e = ensure_smem((const void *)sweep, (size_t)t.M * sizeof(double));
     if (e != cudaSuccess) return e;
     const int grid = items < num_sms ? items : num_sms;
-    k_zfwd_f64<KP, MT><<<grid, kZThreads, Z::kFwdBytes, s>>>(t, w, nb);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_pdl(w.pdl, k_zfwd_f64<KP, MT>, dim3(grid), dim3(kZThreads), Z::kFwdBytes, s, t, w, nb);
+    if (e != cudaSuccess) return e;
     const int mpb = 128 / t.K;   // modes per CTA
-    sweep<<<dim3((t.L + mpb - 1) / mpb, nb), 128, (size_t)t.M * sizeof(double), s>>>(t, w);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_zinv_f64<KP, MT><<<grid, kZThreads, Z::kInvBytes, s>>>(t, w, nb);
-    return cudaGetLastError();
+    e = launch_pdl(w.pdl, sweep, dim3((t.L + mpb - 1) / mpb, nb), dim3(128), (size_t)t.M * sizeof(double), s, t, w);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(w.pdl, k_zinv_f64<KP, MT>, dim3(grid), dim3(kZThreads), Z::kInvBytes, s, t, w, nb);
 }
 
 cudaError_t launch_solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s)
