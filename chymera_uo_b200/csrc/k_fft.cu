@@ -56,12 +56,30 @@ struct Shape {
         for (int i = 0; i <= s; ++i) sp /= radix(i);
         return sp;
     }
+    // rotations of all stages in the compact table
+    static constexpr int compact()
+    {
+        int c = 0;
+        for (int i = 0; i < nst(); ++i) c += span(i);
+        return c;
+    }
 };
 
-template <int L>
+// INV: k_inverse's tile, else k_forward's.  A tile wide enough that the rows
+// a warp reads are whole 128-byte lines, and small enough that two or more
+// CTAs share an SM: the passes over shared memory wait at barriers, which only
+// another CTA can fill.  Measured, us:
+//   k_forward, 16 against 8 columns:  512x128x512 155 / 262, 256x64x1024
+//     130 / 180 (8 columns: half of each line's sectors per request);
+//     16 against 32: 128x64x128 x8 43.9 / 48.1, 256x128x128 24.8 / 27.7,
+//     256x128x256 x2 81 / 101, but 64x32x64 x32 32.4 / 27.7
+//   k_inverse, 16 against 8: 512x128x512 174 / 172, 256x64x1024 132 / 125;
+//     16 against 32: 128x64x128 x8 45.6 / 43.0
+template <int L, bool INV = false>
 struct Tile {
     static constexpr int N = L / 2;
-    static constexpr int TC = L <= 128 ? 32 : (L <= 256 ? 16 : 8);  // columns per CTA
+    static constexpr int TC = INV ? (L <= 128 ? 32 : (L <= 256 ? 16 : 8))   // columns per CTA
+                                  : (L <= 64 ? 32 : 16);
     static constexpr int RS = TC + 2;                               // row stride (doubles, even)
     static constexpr int ROWS = L + 2;
     static constexpr int TPC = 256 / TC;                            // threads per column
@@ -168,8 +186,10 @@ __device__ __forceinline__ void bulk_fft_tables(const FftDev &f, const FftSmem &
 template <int L>
 __host__ __device__ constexpr size_t fft_table_bytes()
 {
-    // twiddles <= N entries x 6 doubles, flags, perm, REALTR (N/2+1) x 2
-    return (size_t)(L / 2) * 6 * 8 + (size_t)(L / 2) + (size_t)(L / 2) * 4 + (size_t)(L / 4 + 1) * 16 + 64;
+    // twiddles (compact entries x 6 doubles), REALTR (N/2+1) x 2, perm, flags
+    // (16-byte pieces), up to a 16-byte boundary
+    constexpr size_t nc = Shape<L / 2>::compact();
+    return nc * 48 + (size_t)(L / 4 + 1) * 16 + (size_t)(L / 2) * 4 + ((nc + 15) & ~(size_t)15);
 }
 
 template <int L>
@@ -178,7 +198,7 @@ __device__ __forceinline__ FftSmem carve_fft(char *p)
     constexpr int N = L / 2;
     FftSmem s;
     s.tw = (double *)p;
-    p += (size_t)N * 6 * 8;
+    p += (size_t)Shape<N>::compact() * 48;
     s.rt = (double *)p;
     p += (size_t)(N / 2 + 1) * 16;
     s.perm = (int *)p;
@@ -235,23 +255,31 @@ __device__ __forceinline__ void butterfly(double &a0, double &b0, double &a1, do
 }
 
 // Stages S and S+1 of the transform in one pass over shared memory (S alone
-// when it is the last).  Stage S+1 works inside the blocks of stage S, so the
-// R_S * R_{S+1} elements base + i H_{S+1} of a group are closed under both
-// stages: a thread loads them, applies stage S's R_{S+1} butterflies and then
+// when it is the last or the two hold more elements than a thread should).
+// Stage S+1 works inside the blocks of stage S, so the R_S * R_{S+1} elements
+// base + i H_{S+1} of a group are closed under both stages: a thread loads them, applies stage S's R_{S+1} butterflies and then
 // stage S+1's R_S butterflies in registers, and stores them back.  Each
 // butterfly is the one the element-by-element stage loop would apply.
 //
 // Layout of the complex element e in the tile (row stride RS): interleaved
 // (Re in row 2e, Im in row 2e+1) or split (Re in row e, Im in row IM0+e).
-template <int L, int S, bool FWD, int RS = Tile<L>::RS, bool SPLIT = false>
+template <int L, int S, bool FWD, int RS, bool SPLIT = false>
 __device__ __forceinline__ void stage_pairs(double *A, const FftSmem &s, const FftDev &f)
 {
-    using T = Tile<L>;
+    using T = Tile<L, !FWD>;
     using Sh = Shape<T::N>;
     auto rre = [](int e) { return SPLIT ? e : 2 * e; };
     auto rim = [](int e) { return SPLIT ? T::IM0 + e : 2 * e + 1; };
     if constexpr (S < Sh::nst()) {
-        constexpr bool two = S + 1 < Sh::nst();
+        // Two radix-4 stages hold 16 complex elements and need ~100 registers,
+        // two CTAs an SM; 8 elements or fewer stay below 64 registers, four
+        // CTAs, for one more pass.  Measured, one pass of 16 against 8, us:
+        //   k_forward L=32 50 / 30, 128 90 / 87, 512 155 / 184, 1024 equal
+        //   k_inverse L=32 41 / 26, 128 90 / 69, 512 228 / 173, 1024 129 / 138
+        // (L=64, 256: no two radix-4 stages stand side by side)
+        constexpr int kMost = L <= (FWD ? 128 : 512) ? 8 : 16;
+        constexpr int RN = Sh::radix(S + 1 < Sh::nst() ? S + 1 : S);
+        constexpr bool two = S + 1 < Sh::nst() && Sh::radix(S) * RN <= kMost;
         constexpr int R1 = Sh::radix(S), H1 = Sh::span(S);
         constexpr int R2 = two ? Sh::radix(S + 1) : 1, H2 = two ? Sh::span(S + 1) : H1;
         constexpr int G = R1 * R2, NG = T::N / G;
@@ -308,7 +336,7 @@ __device__ __forceinline__ void stage_pairs(double *A, const FftSmem &s, const F
 template <int L>
 __device__ __forceinline__ void realtr_pairs(double *A, const FftSmem &s)
 {
-    using T = Tile<L>;
+    using T = Tile<L, true>;
     constexpr int n = T::N, nh = n / 2 + 1, RS = T::TC, I0 = T::IM0;
 #pragma unroll
     for (int it = 0; it < (nh * T::TC + 255) / 256; ++it) {
@@ -497,7 +525,7 @@ __global__ void __launch_bounds__(256) k_forward(DevTables t, BatchPtrs bp, Work
     }
     __syncthreads();
 
-    stage_pairs<L, 0, true>(A, fs, t.fwd);
+    stage_pairs<L, 0, true, T::RS>(A, fs, t.fwd);
 
     // REALTR (pot/fft.f:2-70) on the transform in natural order -- its sample
     // q is row perm[q], and A(N+1) = A(1) (pot/fft.f:44-45) -- with the modes
@@ -752,7 +780,7 @@ template <int L>
 __global__ void __launch_bounds__(256) k_inverse(DevTables t, BatchPtrs bp, Work w, StarDev x, int xmode,
                                                  const __grid_constant__ CUtensorMap xmap)
 {
-    using T = Tile<L>;
+    using T = Tile<L, true>;
     constexpr int n = T::N, RS = T::TC, I0 = T::IM0;
     extern __shared__ __align__(128) char smem_raw[];
     // Split layout, row stride TC: row q holds A1(q+1) = mode q (q = 0..N),
@@ -1128,7 +1156,7 @@ template <int L>
 static cudaError_t inverse_l(const DevTables &t, const BatchPtrs &bp, const Work &w, const StarDev &x, int nb,
                              cudaStream_t s, int *launches)
 {
-    using T = Tile<L>;
+    using T = Tile<L, true>;
     const size_t sm = (size_t)T::ROWSI * T::TC * sizeof(double) + (size_t)(L / 2) * 8 + fft_table_bytes<L>() + 16 +
                       4 * 81 * sizeof(double);   // the weights of NPOINT <= 10
     cudaError_t e = ensure_smem((const void *)k_inverse<L>, sm);
