@@ -351,6 +351,11 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, int bytes
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes)
                  : "memory");
 }
+// the same, 4 bytes
+__device__ __forceinline__ void cp_async4(void *dst, const void *src, int bytes)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -1947,17 +1952,18 @@ __global__ void __launch_bounds__(256, 1) k_mode_pair(DevTables t, Work w, Mixed
 // bytes.  Bound by HBM: 11.4 GB at four solves of 512x128x512 with one
 // correction (1.75 ms at the measured rate).  Measured there, all mode solves:
 // five kernels with residual, scaled rows and update each through memory 6.35
-// ms, now 3.27 (down 0.51 and 1.10, sweeps 0.36 each, up 0.41 and 0.52).  What is
+// ms, now 2.83 (down 0.46 and 0.71, sweeps 0.36 each, up 0.41 and 0.52).  What is
 // left is latency at 16 warps per SM: two CTAs fill registers and shared memory.
 // ---------------------------------------------------------------------------
 constexpr int kWideMaxJ = 1024;  // largest JMAX of the wide pipeline
 constexpr int kWideT = 64;       // columns of a tile: two CTAs per SM, one loading while the other multiplies
 
-// Shared memory of the two product kernels: eigenbasis tile, operand tile (then,
-// in k_wide_up, the staged product), row tables, reductions, barriers.
+// Shared memory of the two product kernels: eigenbasis tile, operand tile (in
+// k_wide_down before that F's tile, in k_wide_up after it the staged product), row
+// tables, reductions, the columns beside F's tile, barriers.
 struct WideSmem {
-    static constexpr int a = 0, b = kAImg, rows = b + kWideT * 512, red = rows + 5 * 128 * 8, bars = red + 32 * 8,
-                         bytes = bars + 64;
+    static constexpr int a = 0, b = kAImg, rows = b + kWideT * 512, red = rows + 5 * 128 * 8, halo = red + 32 * 8,
+                         bars = halo + 256 * 4, bytes = bars + 64;
 };
 
 // Per-CTA state of a product kernel: tensor memory (64 columns), barriers, the
@@ -2086,6 +2092,13 @@ __device__ __forceinline__ uint32_t pack_half2(__half a, __half b)
 // the iterate the residual subtracts: 0 none, 1 F / d_k, 2 xit.  Warp w forms
 // rows 16 w .. 16 w + 15 of columns lane and lane + 32: consecutive k, so that a
 // thread's values are whole 16-byte granules of the operand tile.
+// The next tile is on its way while this one is multiplied: its first eight rows
+// of X in the registers that the operand has left, and (kSrc = 1) its tile of F
+// -- 32 KB, as many as the operand's -- in the operand's place once the product
+// has read it.  Measured at four solves of 512x128x512, kSrc = 1: with all loads
+// at the tile's start 1.13 ms; the boundary column's values in one load per lane
+// instead of one per row (which only the edge tiles waited for) 0.82; F staged
+// and the first rows ahead 0.71 (0.51, 0.46 and 0.46 without an iterate).
 template <int kSrc>
 __global__ void __launch_bounds__(256, 2) k_wide_down(DevTables t, Work w, MixedDev x, WideDev d, int tiles)
 {
@@ -2095,14 +2108,64 @@ __global__ void __launch_bounds__(256, 2) k_wide_down(DevTables t, Work w, Mixed
     wide_setup(c, sm, t, x);
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, M = t.M, NZ = t.NZ, J = t.JX, k0 = 16 * warp;
+    float *sF = reinterpret_cast<float *>(c.sBh);                     // [128][64]
+    float *sH = reinterpret_cast<float *>(sm + WideSmem::halo);       // [2][128]: the columns beside the tile
+
+    // F's tile and the columns beside it into sF and sH; rows from NZ and columns
+    // from M on are zeros
+    auto load_f = [&](int tile) {
+        const int item = tile / d.nt, j0 = (tile - item * d.nt) * kWideT;
+        const float *Fl = d.F + (size_t)item * d.sx;
+        if ((t.J & 3) == 0) {
+            const int q = 4 * (threadIdx.x & 15), k1 = threadIdx.x >> 4;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int k = k1 + 16 * i;
+                const int nq = k < NZ ? min(max(M - j0 - q, 0), 4) : 0;
+                cp_async16(sF + k * kWideT + q, nq > 0 ? Fl + (size_t)k * t.J + j0 + q : Fl, 4 * nq);
+            }
+        } else {   // rows off the 16-byte boundaries
+            const int q = threadIdx.x & 63, k1 = threadIdx.x >> 6;
+#pragma unroll 8
+            for (int i = 0; i < 32; ++i) {
+                const int k = k1 + 4 * i;
+                const bool on = k < NZ && j0 + q < M;
+                cp_async4(sF + k * kWideT + q, on ? Fl + (size_t)k * t.J + j0 + q : Fl, on ? 4 : 0);
+            }
+        }
+        const int k = threadIdx.x & 127, jh = threadIdx.x < 128 ? j0 - 1 : j0 + kWideT;
+        const bool on = k < NZ && jh >= 0 && jh < M;
+        cp_async4(sH + threadIdx.x, on ? Fl + (size_t)k * t.J + jh : Fl, on ? 4 : 0);
+        cp_async_commit();
+    };
+
+    // X's rows k0 .. k0 + 7 (past row NZ: that row again, dropped below) and, in
+    // lane i of the tile of column M-1, the outer boundary's value of row k0 + i
+    double y[2][8], ye = 0.0;
+    auto load_x = [&](int tile) {
+        const int item = tile / d.nt, j0 = (tile - item * d.nt) * kWideT;
+        const double *Xl = w.X + (size_t)item * t.K * J;   // X's solves are L * K * J apart
+        const int ja = min(j0 + lane, t.J - 1), jb = min(j0 + lane + 32, t.J - 1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const double *px = Xl + (size_t)min(k0 + i, NZ) * J;
+            y[0][i] = px[ja];
+            y[1][i] = px[jb];
+        }
+        if (j0 + kWideT >= M) ye = Xl[(size_t)min(k0 + (lane & 15), NZ) * J + M];
+    };
+
+    if ((int)blockIdx.x < tiles) {
+        load_x(blockIdx.x);
+        if constexpr (kSrc == 1) load_f(blockIdx.x);
+    }
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int item = tile / d.nt, j0 = (tile - item * d.nt) * kWideT;
         const int l = item % t.L, m = l <= t.N ? l : l - t.N;
         const double xl2 = 2.0 * (t.xlamm[m] - 1.0);
-        const double *Xl = w.X + (size_t)item * t.K * J;   // X's solves are L * K * J apart
-        const float *Fl = d.F + (size_t)item * d.sx;
-        const double *xl = d.xit + (size_t)item * d.sx;
-        if (tile + (int)gridDim.x < tiles) {   // the next tile: KMAX rows of 512 bytes of X, 256 of F
+        const double *Xl = w.X + (size_t)item * t.K * J;
+        const bool more = tile + (int)gridDim.x < tiles;
+        if (more) {   // the next tile: KMAX rows of 512 bytes of X, 256 of F
             const int nt = tile + gridDim.x, ni = nt / d.nt, nj = (nt - ni * d.nt) * kWideT;
             for (int i = threadIdx.x; i < 4 * t.K; i += 256)
                 if (nj + 16 * (i & 3) < J) l2_prefetch(w.X + ((size_t)ni * t.K + (i >> 2)) * J + nj + 16 * (i & 3));
@@ -2131,108 +2194,112 @@ __global__ void __launch_bounds__(256, 2) k_wide_down(DevTables t, Work w, Mixed
         // into the arrays (a load under a condition waits for the ones before
         // it): what lies outside the interior meets zero coefficients (AN(1),
         // CN(NZ), AM(1), CM(M), the columns past M) or is dropped below.
-        using XT = std::conditional_t<kSrc == 2, double, float>;
         const int ja = min(j0 + lane, t.J - 1), jb = min(j0 + lane + 32, t.J - 1);
-        const int jh = lane == 31 ? min(j0 + kWideT, t.J - 1) : max(j0 - 1, 0);   // the halo column (lanes 0 and 31)
         const bool in[2] = {j0 + lane < M, j0 + lane + 32 < M};
-        const XT *it0 = nullptr;
-        if constexpr (kSrc == 1) it0 = Fl;
-        if constexpr (kSrc == 2) it0 = xl;
-        auto scaled = [&](XT f, int k) -> XT {
-            if constexpr (kSrc == 2) return f * c.cd[k].y;
-            else return f;
-        };
-        // the top boundary row, for the warp that holds row NZ
-        const int itop = NZ - 1 - k0;
-        double top[2] = {0.0, 0.0};
-        if (itop >= 0 && itop < 16) {
-            top[0] = Xl[(size_t)NZ * J + ja];
-            top[1] = Xl[(size_t)NZ * J + jb];
-        }
+        const bool edge = j0 + kWideT >= M;   // the tile of column M-1 (or past it)
+        const int itop = NZ - 1 - k0;         // the row under the top boundary, in the warp that holds it
         float v[2][16];
         float vmax = 0.0f;
-        XT mid[2] = {};
+        const double *px = Xl + (size_t)min(k0 + 8, NZ) * J;   // the rows after y's
         double up[2] = {}, mi[2] = {};   // rows k-1 and k in FP64
-        const int kf = min(k0, NZ - 1);
-        const double *px = Xl + (size_t)kf * J;
-        const XT *pi = it0 + (size_t)kf * t.J;
-        if constexpr (kSrc != 0) {
-            const XT *pu = it0 + (size_t)min(max(k0 - 1, 0), NZ - 1) * t.J;
-            const XT u0 = pu[ja], u1 = pu[jb], m0 = pi[ja], m1 = pi[jb];
-            up[0] = (double)scaled(u0, max(k0 - 1, 0));
-            up[1] = (double)scaled(u1, max(k0 - 1, 0));
-            mid[0] = scaled(m0, k0);
-            mid[1] = scaled(m1, k0);
-            mi[0] = (double)mid[0];
-            mi[1] = (double)mid[1];
+        // kSrc = 2: a batch of xit's rows below and of the halo column (lanes 0 and 31)
+        double dn[2][8], halo[8];
+        const double *pi = d.xit + (size_t)item * d.sx + (size_t)min(k0, NZ - 1) * t.J;
+        const int jh = lane == 31 ? min(j0 + kWideT, t.J - 1) : max(j0 - 1, 0);
+        if constexpr (kSrc == 2) {
+            const double *pu = d.xit + (size_t)item * d.sx + (size_t)min(max(k0 - 1, 0), NZ - 1) * t.J;
+            const double u0 = pu[ja], u1 = pu[jb], m0 = pi[ja], m1 = pi[jb];
+            up[0] = u0 * c.cd[max(k0 - 1, 0)].y;
+            up[1] = u1 * c.cd[max(k0 - 1, 0)].y;
+            mi[0] = m0 * c.cd[k0].y;
+            mi[1] = m1 * c.cd[k0].y;
         }
-        const bool edge = j0 + kWideT >= M;   // the tile of column M-1 (or past it)
+        // kSrc = 1: this thread's cells and their neighbours in the staged tile
+        const float *fr = sF + k0 * kWideT + lane;
+        const float *fl = lane == 0 ? sH + k0 : fr - 1, *fh = lane == 31 ? sH + 128 + k0 : fr + 33;
+        const int sl = lane == 0 ? 1 : kWideT, sh = lane == 31 ? 1 : kWideT;
+        if constexpr (kSrc == 1) {
+            cp_async_wait<0>();
+            __syncthreads();
+            const float *fu = k0 > 0 ? fr - kWideT : fr;
+            up[0] = (double)fu[0];
+            up[1] = (double)fu[32];
+            mi[0] = (double)fr[0];
+            mi[1] = (double)fr[32];
+        }
 #pragma unroll
-        for (int i0 = 0; i0 < 16; i0 += 8) {
-            // this batch's loads: X, the rows below, the halo columns (lane 0: the
-            // one before the tile, lane 31: the one after)
-            double y[2][8];
-            XT dn[2][8], halo[8];
+        for (int i = 0; i < 16; ++i) {
+            const int k = k0 + i, i8 = i & 7;
+            if constexpr (kSrc == 2)
+                if (i8 == 0) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+                    for (int u = 0; u < 8; ++u) {
+                        halo[u] = pi[jh];
+                        if (k + u < NZ - 1) pi += t.J;   // uniform; rows NZ and past repeat the last one
+                        dn[0][u] = pi[ja];
+                        dn[1][u] = pi[jb];
+                    }
+                }
+            const double2 ba = c.ba[k], cd = c.cd[k];
+            // 4 pi G rho with the boundary folds (pot/pot3.f:212-224); the row
+            // above the last one is the top boundary's
+            const double pg = t.pig4 * cd.y;
+            double r[2] = {pg * y[0][i8], pg * y[1][i8]};
+            if (i == itop) {
+                r[0] = r[0] - t.cnmax * cd.y * y[0][(i + 1) & 7];
+                r[1] = r[1] - t.cnmax * cd.y * y[1][(i + 1) & 7];
+            }
+            if (edge) {
+                const double yM = t.cmmax * cd.y * __shfl_sync(0xffffffffu, ye, i);
+                if (j0 + lane == M - 1) r[0] = r[0] - yM;
+                if (j0 + lane + 32 == M - 1) r[1] = r[1] - yM;
+            }
+            if (i < 8) {   // row k + 8 takes its place
                 y[0][i] = px[ja];
                 y[1][i] = px[jb];
-                if constexpr (kSrc != 0) halo[i] = pi[jh];
-                if (k0 + i0 + i < NZ - 1) {   // uniform; rows NZ and past repeat the last one
-                    px += J;
-                    pi += t.J;
-                }
-                if constexpr (kSrc != 0) {
-                    dn[0][i] = pi[ja];
-                    dn[1][i] = pi[jb];
-                }
+                if (k + 8 < NZ) px += J;
             }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int k = k0 + i0 + i;
-                const double2 ba = c.ba[k], cd = c.cd[k];
-                // 4 pi G rho with the boundary folds (pot/pot3.f:212-224)
-                const double pg = t.pig4 * cd.y;
-                double r[2] = {pg * y[0][i], pg * y[1][i]};
-                if (i0 + i == itop) {
-                    r[0] = r[0] - t.cnmax * cd.y * top[0];
-                    r[1] = r[1] - t.cnmax * cd.y * top[1];
-                }
-                if (edge) {
-                    const double yM = t.cmmax * cd.y * Xl[(size_t)min(k, NZ - 1) * J + M];
-                    if (j0 + lane == M - 1) r[0] = r[0] - yM;
-                    if (j0 + lane + 32 == M - 1) r[1] = r[1] - yM;
-                }
-                if constexpr (kSrc != 0) {
-                    const XT hv = scaled(halo[i], k);
-                    const XT l0 = __shfl_sync(0xffffffffu, mid[0], lane + 31), l1 = __shfl_sync(0xffffffffu, mid[1], lane + 31);
-                    const XT r0 = __shfl_sync(0xffffffffu, mid[0], lane + 1), r1 = __shfl_sync(0xffffffffu, mid[1], lane + 1);
-                    const XT lf[2] = {lane == 0 ? hv : l0, lane == 0 ? l0 : l1};
-                    const XT rt[2] = {lane == 31 ? r1 : r0, lane == 31 ? hv : r1};
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const XT nx = scaled(dn[h][i], min(k + 1, 127));
-                        const double below = (double)nx;
-                        double ax = (ba.x + bm[h]) * mi[h];
-                        ax += ba.y * up[h];
-                        ax += cd.x * below;
-                        ax += am[h] * (double)lf[h];
-                        ax += cm[h] * (double)rt[h];
-                        r[h] = r[h] - ax;
-                        up[h] = mi[h];
-                        mi[h] = below;
-                        mid[h] = nx;
-                    }
+            if constexpr (kSrc != 0) {
+                double below[2], lf[2], rt[2];
+                if constexpr (kSrc == 1) {
+                    const float *fd = i < 15 ? fr + (i + 1) * kWideT : fr + (k < 127 ? 16 : 15) * kWideT;
+                    below[0] = (double)fd[0];
+                    below[1] = (double)fd[32];
+                    lf[0] = (double)fl[i * sl];
+                    lf[1] = (double)fr[i * kWideT + 31];
+                    rt[0] = (double)fr[i * kWideT + 1];
+                    rt[1] = (double)fh[i * sh];
+                } else {
+                    const double hv = halo[i8] * cd.y, dkn = c.cd[min(k + 1, 127)].y;
+                    const double l0 = __shfl_sync(0xffffffffu, mi[0], lane + 31), l1 = __shfl_sync(0xffffffffu, mi[1], lane + 31);
+                    const double r0 = __shfl_sync(0xffffffffu, mi[0], lane + 1), r1 = __shfl_sync(0xffffffffu, mi[1], lane + 1);
+                    below[0] = dn[0][i8] * dkn;
+                    below[1] = dn[1][i8] * dkn;
+                    lf[0] = lane == 0 ? hv : l0;
+                    lf[1] = lane == 0 ? l0 : l1;
+                    rt[0] = lane == 31 ? r1 : r0;
+                    rt[1] = lane == 31 ? hv : r1;
                 }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const float f = in[h] && k < NZ ? (float)r[h] : 0.0f;
-                    v[h][i0 + i] = f;
-                    vmax = fmaxf(vmax, fabsf(f));
+                    double ax = (ba.x + bm[h]) * mi[h];
+                    ax += ba.y * up[h];
+                    ax += cd.x * below[h];
+                    ax += am[h] * lf[h];
+                    ax += cm[h] * rt[h];
+                    r[h] = r[h] - ax;
+                    up[h] = mi[h];
+                    mi[h] = below[h];
                 }
             }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float f = in[h] && k < NZ ? (float)r[h] : 0.0f;
+                v[h][i] = f;
+                vmax = fmaxf(vmax, fabsf(f));
+            }
         }
-        const float s = pow2_scale(wide_max(c, vmax));
+        const float s = pow2_scale(wide_max(c, vmax));   // also: the staged tile has been read
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -2249,7 +2316,10 @@ __global__ void __launch_bounds__(256, 2) k_wide_down(DevTables t, Work w, Mixed
                 *reinterpret_cast<uint4 *>(c.sBh + o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                 *reinterpret_cast<uint4 *>(c.sBl + o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
+        if (more) load_x(tile + gridDim.x);
         const bool ok = wide_product(c, false);
+        if constexpr (kSrc == 1)
+            if (more) load_f(tile + gridDim.x);
         float *dst = d.W + (size_t)item * d.sw + (size_t)(j0 + 32 * (warp >> 2)) * 128 + 32 * (warp & 3) + lane;
         const float unscale = 1.0f / (kAScale * s);
         float o[32];
