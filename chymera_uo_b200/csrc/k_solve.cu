@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(128) k_thomas_table(DevTables t, double *rec, 
 // second register set at constant offsets (KC = KMAX; 0: KMAX known at run time
 // only); AM is staged in shared memory (the streaming loads evict it from L1).
 // At 8 solves of 256x128x256: 0.53 ms with the divisions, 0.345 ms now, about
-// the time of its 330 MB per solve; with an eight-byte cp.async ring three
+// the time of its 330 MB per solve (W read and written twice); with an eight-byte cp.async ring three
 // chunks deep instead of the registers 0.54 ms (bound by the copies' issue).
 template <int KC>
 __global__ void __launch_bounds__(128) k_thomas_f64(DevTables t, Work w)
@@ -278,6 +278,208 @@ __global__ void __launch_bounds__(128) k_thomas_f64(DevTables t, Work w)
         if (c + 2 < nf) load_up(ya, ta);
         if (c + 1 < nf) up(yb, tb);
     }
+}
+
+// The same sweeps with the eliminated rows on chip, for grids of at most 256 rows
+// and KMAX >= 32: the 128 threads of a CTA own the 128 lanes of tensor memory,
+// whose 512 columns hold a lane's M <= 256 FP64 values, so W is read once and
+// written once.  One persistent CTA per SM walks the groups of 128 / K modes; W
+// and the table rows arrive as bulk copies, sixteen rows (32 KB) a slot, kTmSlots
+// slots ahead, also across groups: the next group's rows are on their way while
+// this one substitutes back and stores.  Bound by HBM and the table's L2 reads.
+// The recurrences, and so the bits, are k_thomas_f64's.  Eight solves of
+// 256x128x256: 0.352 -> 0.228 ms (4.7 TB/s of W alone), 0.286 with the groups
+// solve by solve (each solve's pass over the 67 MB of table evicts it).
+constexpr int kTmSlots = 6, kTmRows = 16;
+constexpr size_t kTmSlotDoubles = 2 * kTmRows * 128;
+constexpr size_t kTmBytes = kTmSlots * kTmSlotDoubles * 8 + 256 * 8 + kTmSlots * 8 + 16;
+
+__device__ __forceinline__ uint32_t tm_sm32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// bounded wait on phase `parity`: false after it ran out
+__device__ __forceinline__ bool tm_bar_wait(uint64_t *bar, uint32_t parity)
+{
+    for (long long i = 0; i < (1ll << 26); ++i) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done)
+                     : "r"(tm_sm32(bar)), "r"(parity)
+                     : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+__device__ __forceinline__ void tm_bulk(double *dst, const double *src, uint32_t bytes, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tm_sm32(dst)),
+                 "l"(src), "r"(bytes), "r"(tm_sm32(bar))
+                 : "memory");
+}
+
+// eight FP64 values (sixteen columns) of this thread's lane
+__device__ __forceinline__ void tm_put8(uint32_t ta, const double *v)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(ta),
+                 "r"(__double2loint(v[0])), "r"(__double2hiint(v[0])), "r"(__double2loint(v[1])), "r"(__double2hiint(v[1])),
+                 "r"(__double2loint(v[2])), "r"(__double2hiint(v[2])), "r"(__double2loint(v[3])), "r"(__double2hiint(v[3])),
+                 "r"(__double2loint(v[4])), "r"(__double2hiint(v[4])), "r"(__double2loint(v[5])), "r"(__double2hiint(v[5])),
+                 "r"(__double2loint(v[6])), "r"(__double2hiint(v[6])), "r"(__double2loint(v[7])), "r"(__double2hiint(v[7]))
+                 : "memory");
+}
+__device__ __forceinline__ void tm_get8(uint32_t ta, double *v)
+{
+    int r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(ta)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __hiloint2double(r[2 * i + 1], r[2 * i]);
+}
+
+template <int K>
+__global__ void __launch_bounds__(128, 1) k_thomas_tm(DevTables t, Work w, int groups)
+{
+    constexpr int R = kTmRows, G = 128 / K;   // rows of a slot, modes of a group
+    extern __shared__ __align__(128) double tsm[];
+    double *am = tsm + kTmSlots * kTmSlotDoubles;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(am + 256);
+    uint32_t *slot = reinterpret_cast<uint32_t *>(bar + kTmSlots);
+    const int tid = threadIdx.x, p = tid % K, g = tid / K, M = t.M, nc = (M + R - 1) / R, gl = t.L / G;
+    pdl_go();
+    if (tid == 0) {
+        for (int i = 0; i < kTmSlots; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tm_sm32(bar + i)));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int j = tid; j < M; j += 128) am[j] = t.am[j];
+    pdl_wait();
+    // tensor memory only once nothing is waited for that another kernel does
+    if (tid < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tm_sm32(slot)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tm = *slot + ((uint32_t)(tid & 96) << 16);
+
+    // group i is solve b's modes l0 ..: all solves' groups of the same table rows, of
+    // both halves of the modes (m = l and l - N), one after the other, so that the
+    // table comes from memory once
+    const int per = 2 * (groups / gl);
+    auto place = [&](int i, int &b, int &l0) {
+        const int q = i / per, r = i - q * per;
+        b = r >> 1;
+        l0 = (q + (r & 1) * (gl / 2)) * G;
+    };
+
+    // the copies, in the order of their use: per group the chunks of W and the
+    // pivot reciprocals upwards, then the multipliers' downwards (thread 0)
+    int pg = blockIdx.x, ps = 0, pslot = 0, fills = 0;
+    auto issue = [&]() {
+        if (pg >= groups) return;
+        const int c = ps < nc ? ps : 2 * nc - 1 - ps, rows = min(R, M - c * R);
+        int b, l0;
+        place(pg, b, l0);
+        const uint32_t bytes = (uint32_t)(rows * K * 8);
+        double *d = tsm + pslot * kTmSlotDoubles;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tm_sm32(bar + pslot)),
+                     "r"(bytes * G * (ps < nc ? 2u : 1u))
+                     : "memory");
+        for (int q = 0; q < G; ++q) {
+            const size_t tab = ((size_t)mode_m(l0 + q, t.N) * M + c * R) * K;
+            if (ps < nc) {
+                tm_bulk(d + q * R * K, w.W + (size_t)b * w.sW + ((size_t)(l0 + q) * t.J + c * R) * K, bytes, bar + pslot);
+                tm_bulk(d + R * 128 + q * R * K, t.th_rec + tab, bytes, bar + pslot);
+            } else {
+                tm_bulk(d + R * 128 + q * R * K, t.th_mul + tab, bytes, bar + pslot);
+            }
+        }
+        ++fills;
+        pslot = pslot + 1 == kTmSlots ? 0 : pslot + 1;
+        if (++ps == 2 * nc) {
+            ps = 0;
+            pg += gridDim.x;
+        }
+    };
+    if (tid == 0)
+        for (int i = 0; i < kTmSlots; ++i) issue();
+
+    int cs = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    auto next = [&]() {   // this chunk's slot has been read: refill it
+        __syncthreads();
+        if (tid == 0 && ok) issue();
+        if (++cs == kTmSlots) {
+            cs = 0;
+            ph ^= 1u;
+        }
+    };
+    for (int gr = blockIdx.x; gr < groups; gr += gridDim.x) {
+        int b, l;
+        place(gr, b, l);
+        l += g;
+        double *Wp = w.W + (size_t)b * w.sW + (size_t)l * t.J * K + p;
+        double prev = 0.0;
+        for (int c = 0; c < nc; ++c) {
+            ok = ok && tm_bar_wait(bar + cs, ph);
+            const double *y = tsm + cs * kTmSlotDoubles + g * R * K + p, *r = y + R * 128;
+            double v[R];
+            const int rows = M - c * R;
+            if (rows >= R) {
+#pragma unroll
+                for (int i = 0; i < R; ++i) v[i] = prev = (y[i * K] - am[c * R + i] * prev) * r[i * K];
+            } else {
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    if (i < rows) prev = (y[i * K] - am[c * R + i] * prev) * r[i * K];
+                    v[i] = prev;
+                }
+            }
+            tm_put8(tm + c * 2 * R, v);
+            tm_put8(tm + c * 2 * R + 16, v + 8);
+            next();
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        double x = ok ? prev : __longlong_as_double(0x7ff8000000000000ll);   // a copy that never came
+        for (int c = nc - 1; c >= 0; --c) {
+            double v[R];
+            tm_get8(tm + c * 2 * R, v);
+            tm_get8(tm + c * 2 * R + 16, v + 8);
+            ok = ok && tm_bar_wait(bar + cs, ph);
+            const double *m = tsm + cs * kTmSlotDoubles + R * 128 + g * R * K + p;
+            double *o = Wp + (size_t)c * R * K;
+            const int last = M - 1 - c * R;   // the last row's place in its chunk: x as it is
+            if (!ok) x = __longlong_as_double(0x7ff8000000000000ll);
+            if (last >= R) {
+#pragma unroll
+                for (int i = R - 1; i >= 0; --i) {
+                    x = v[i] - m[i * K] * x;
+                    if (p < t.NZ) o[i * K] = x;
+                }
+            } else {
+#pragma unroll
+                for (int i = R - 1; i >= 0; --i) {
+                    if (i < last) x = v[i] - m[i * K] * x;
+                    if (i <= last && p < t.NZ) o[i * K] = x;
+                }
+            }
+            next();
+        }
+    }
+    // a wait that ran out: every slot's last copy (bounded) before the memory goes
+    if (tid == 0 && !ok)
+        for (int i = 0; i < kTmSlots; ++i) {
+            const int f = fills / kTmSlots + (i < fills % kTmSlots ? 1 : 0);
+            if (f > 0) tm_bar_wait(bar + i, (uint32_t)(f - 1) & 1u);
+        }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(*slot));
 }
 
 // X_l(j,k) = sum_p V(k,p) W[l][j][p] for the interior (k < NZ, j < M).  A tile
@@ -374,7 +576,24 @@ static cudaError_t solve_fp64(const DevTables &t, const Work &w, int nb, int num
     e = launch_pdl(w.pdl, k_zfwd_f64<KP, MT>, dim3(grid), dim3(kZThreads), Z::kFwdBytes, s, t, w, nb);
     if (e != cudaSuccess) return e;
     const int mpb = 128 / t.K;   // modes per CTA
-    e = launch_pdl(w.pdl, sweep, dim3((t.L + mpb - 1) / mpb, nb), dim3(128), (size_t)t.M * sizeof(double), s, t, w);
+    const int groups = t.L / mpb * nb;
+    // k_thomas_tm holds an SM with four warps.  While the groups do not outnumber
+    // the SMs its chain is the shorter one (us, k_thomas_tm / k_thomas_f64): one
+    // solve of 64x32x64 11.0 / 15.8, 128x64x128 14.0 / 24.8, 256x64x64 22.9 / 39.7,
+    // 128x128x128 14.0 / 25.9.  Beyond that it wins by the traffic that it saves
+    // where W and the table outgrow L2: 256x128x256 37 / 56, eight 228 / 352; but
+    // 256x64x128 x4 43.1 / 43.7, 128x64x128 x8 42 / 37, 64x32x64 x32 31 / 21,
+    // 200x32x128 x8 48 / 33 (short chains want more warps, narrow groups more copies).
+    bool on_chip = false;
+    if constexpr (KP >= 32) on_chip = t.K == KP && t.M <= 256 && t.L % (2 * mpb) == 0 && (groups <= num_sms || (KP == 128 && t.M > 128));
+    if constexpr (KP >= 32)
+        if (on_chip) {
+            e = ensure_smem((const void *)k_thomas_tm<KP>, kTmBytes);
+            if (e == cudaSuccess)
+                e = launch_pdl(w.pdl, k_thomas_tm<KP>, dim3(groups < num_sms ? groups : num_sms), dim3(128), kTmBytes, s, t, w, groups);
+        }
+    if (!on_chip)
+        e = launch_pdl(w.pdl, sweep, dim3((t.L + mpb - 1) / mpb, nb), dim3(128), (size_t)t.M * sizeof(double), s, t, w);
     if (e != cudaSuccess) return e;
     return launch_pdl(w.pdl, k_zinv_f64<KP, MT>, dim3(grid), dim3(kZThreads), Z::kInvBytes, s, t, w, nb);
 }
