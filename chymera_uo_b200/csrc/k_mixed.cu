@@ -1952,7 +1952,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_pair(DevTables t, Work w, Mixed
 // bytes.  Bound by HBM: 11.4 GB at four solves of 512x128x512 with one
 // correction (1.75 ms at the measured rate).  Measured there, all mode solves:
 // five kernels with residual, scaled rows and update each through memory 6.35
-// ms, now 2.83 (down 0.46 and 0.71, sweeps 0.36 each, up 0.41 and 0.52).  What is
+// ms, now 2.68 (down 0.46 and 0.71, sweeps 0.285 each, up 0.41 and 0.52).  What is
 // left is latency at 16 warps per SM: two CTAs fill registers and shared memory.
 // ---------------------------------------------------------------------------
 constexpr int kWideMaxJ = 1024;  // largest JMAX of the wide pipeline
@@ -2547,6 +2547,179 @@ __global__ void __launch_bounds__(256) k_wide_sweep(DevTables t, MixedDev x, Wid
     }
 }
 
+// The same sweeps for M <= 512 with the eliminated rows on chip: 128 lanes and 512
+// columns of tensor memory hold an item's 128 x M FP32 values (lane p, the upper
+// half's rows in columns [0, h), the lower half's from h on in the order of its
+// elimination), so W is read once and written once.  One persistent CTA per SM
+// walks the items in k_wide_sweep's order; both halves' rows of W and the table
+// arrive as bulk copies, sixteen rows of each (32 KB) a slot, kSwSlots slots ahead,
+// also across items.  The recurrences, and so the bits, are k_wide_sweep's.  Sweeps of four
+// solves of 512x128x512 0.365 -> 0.285 ms (1.07 GB of W: 0.164 at the measured HBM
+// rate), the four-solve call 4.14 -> 3.98; what is left is the two chains of 256
+// rows at two warps a scheduler.
+constexpr int kSwSlots = 6, kSwRows = 16, kSwHalf = 2 * kSwRows * 128;   // floats of a half's part of a slot
+struct SwSmem {
+    static constexpr int tab = kSwSlots * 2 * kSwHalf * 4, meet = tab + 512 * 4, bars = meet + 256 * 4,
+                         bytes = bars + kSwSlots * 8 + 16;
+};
+
+__global__ void __launch_bounds__(256, 1) k_wide_sweep_tm(DevTables t, MixedDev x, WideDev d, int items)
+{
+    extern __shared__ __align__(1024) uint8_t sm[];
+    constexpr int R = kSwRows;
+    float *ring = reinterpret_cast<float *>(sm), *s_tab = reinterpret_cast<float *>(sm + SwSmem::tab);
+    float *meet = reinterpret_cast<float *>(sm + SwSmem::meet);   // [2][128]
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + SwSmem::bars);
+    uint32_t *slot = reinterpret_cast<uint32_t *>(bar + kSwSlots);
+    const int tid = threadIdx.x, p = tid & 127, M = t.M, NTs = x.ntile;
+    const bool low = tid >= 128;   // the bottom-up half
+    const int h = 32 * ((M + 63) / 64), nc = h / R, ML = M - h;   // ML <= h rows in the lower half
+    pdl_go();
+    if (tid == 0) {
+        for (int i = 0; i < kSwSlots; ++i) mbar_init(bar + i, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int j = tid; j < M; j += 256) s_tab[j] = (float)(j < h ? t.am[j] : t.cm[j]);
+    pdl_wait();
+    // tensor memory only once nothing is waited for that another kernel does
+    if (tid < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(slot)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tm = *slot + ((uint32_t)(tid & 96) << 16) + (low ? h : 0);
+
+    const int nb = items / t.L;
+    auto place = [&](int i, int &item, int &m) {   // k_wide_sweep's order
+        const int q = i / nb, b = i - q * nb, l = (q & 1) ? (q >> 1) + t.N : (q >> 1);
+        item = b * t.L + l;
+        m = l <= t.N ? l : l - t.N;
+    };
+    // the copies in the order of their use: an item's chunks of W and the pivots
+    // from the ends to the meeting rows, then the multipliers' back (thread 0).  A
+    // short chunk of the lower half fills the end of its place.
+    int pi = blockIdx.x, ps = 0, pslot = 0, fills = 0;
+    auto issue = [&]() {
+        if (pi >= items) return;
+        int item, m;
+        place(pi, item, m);
+        const bool down = ps < nc;
+        const int c = down ? ps : 2 * nc - 1 - ps, r2 = max(min(R, ML - c * R), 0), top = c * R, bot = M - c * R - r2;
+        const float *tb = (down ? x.sw_piv : x.sw_mul) + (size_t)m * NTs * 128, *W = d.W + (size_t)item * d.sw;
+        float *u = ring + pslot * 2 * kSwHalf, *v = u + kSwHalf + (R - r2) * 128;
+        mbar_expect_tx(bar + pslot, (uint32_t)(R + r2) * 512u * (down ? 2u : 1u));
+        if (down) bulk_g2s(u, W + (size_t)top * 128, R * 512, bar + pslot);
+        bulk_g2s(u + R * 128, tb + (size_t)top * 128, R * 512, bar + pslot);
+        if (r2 > 0) {
+            if (down) bulk_g2s(v, W + (size_t)bot * 128, r2 * 512, bar + pslot);
+            bulk_g2s(v + R * 128, tb + (size_t)bot * 128, r2 * 512, bar + pslot);
+        }
+        ++fills;
+        pslot = pslot + 1 == kSwSlots ? 0 : pslot + 1;
+        if (++ps == 2 * nc) {
+            ps = 0;
+            pi += gridDim.x;
+        }
+    };
+    if (tid == 0)
+        for (int i = 0; i < kSwSlots; ++i) issue();
+    int cs = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    auto next = [&]() {   // this chunk's slot has been read: refill it
+        __syncthreads();
+        if (tid == 0 && ok) issue();
+        if (++cs == kSwSlots) {
+            cs = 0;
+            ph ^= 1u;
+        }
+    };
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+        int item, m;
+        place(it, item, m);
+        float *W = d.W + (size_t)item * d.sw + p;
+        const float *mul = x.sw_mul + (size_t)m * NTs * 128 + p;
+        const float et = __ldg(mul + (size_t)(h - 1) * 128), fu = __ldg(mul + (size_t)h * 128);
+        float yp = 0.0f;
+        for (int c = 0; c < nc; ++c) {
+            ok = ok && mbar_wait(bar + cs, ph);
+            // the i-th row of the elimination is at i * 128 (upper) or (R-1-i) * 128
+            const float *y = ring + cs * 2 * kSwHalf + p, *co = s_tab + c * R;
+            const int n = low ? ML - c * R : R;
+            float v[R];
+            if (!low) {
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const float rr = y[(R + i) * 128];
+                    v[i] = yp = fmaf(-(co[i] * rr), yp, y[i * 128] * rr);
+                }
+            } else {
+                y += kSwHalf;
+                co = s_tab + M - 1 - c * R;
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    if (i < n) {   // uniform
+                        const float rr = y[(2 * R - 1 - i) * 128];
+                        yp = fmaf(-(co[-i] * rr), yp, y[(R - 1 - i) * 128] * rr);
+                    }
+                    v[i] = yp;
+                }
+            }
+            tm_st16_nw(tm + c * R, v);
+            next();
+        }
+        tm_wait_st();
+        if (!ok) yp = __int_as_float(0x7fc00000);   // a copy that never came
+        meet[(low ? 128 : 0) + p] = yp;
+        __syncthreads();
+        const float yt = meet[p], yu = meet[128 + p];
+        const float xt = (yt + (1.0f - et) * yu) / ((et + fu) - et * fu);
+        const float xu = yu + (1.0f - fu) * xt;
+        float xn = low ? xu : xt;   // the meeting row, then back over this half's rows
+        const bool live = p < t.NZ;
+        for (int c = nc - 1; c >= 0; --c) {
+            float v[R];
+            tm_ld16(tm + c * R, v);
+            ok = ok && mbar_wait(bar + cs, ph);
+            if (!ok) xn = __int_as_float(0x7fc00000);
+            const float *e = ring + cs * 2 * kSwHalf + p;
+            const int n = low ? min(ML - c * R, R) : R;
+            const int last = low ? ML - 1 - c * R : h - 1 - c * R;   // the meeting row's place, if in this chunk
+            if (!low) {
+                float *o = W + (size_t)c * R * 128;
+#pragma unroll
+                for (int i = R - 1; i >= 0; --i) {
+                    if (i != last) xn = v[i] + (1.0f - e[(R + i) * 128]) * xn;
+                    if (live) o[i * 128] = xn;
+                }
+            } else {
+                e += kSwHalf;
+                float *o = W + (ptrdiff_t)(M - 1 - c * R) * 128;
+#pragma unroll
+                for (int i = R - 1; i >= 0; --i)
+                    if (i < n) {
+                        if (i != last) xn = v[i] + (1.0f - e[(2 * R - 1 - i) * 128]) * xn;
+                        if (live) o[-i * 128] = xn;
+                    }
+            }
+            next();
+        }
+    }
+    if (!ok) {   // a wait that ran out: every slot's last copy (bounded) before the memory goes
+        atomicExch(x.err, 1);
+        if (tid == 0)
+            for (int i = 0; i < kSwSlots; ++i) {
+                const int f = fills / kSwSlots + (i < fills % kSwSlots ? 1 : 0);
+                if (f > 0) mbar_wait(bar + i, (uint32_t)(f - 1) & 1u);
+            }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (tid < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(*slot));
+}
+
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
@@ -2806,7 +2979,16 @@ static int wide_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
                  : it == 1 ? wide_launch(k_wide_down<1>, p, tiles, s)
                            : wide_launch(k_wide_down<2>, p, tiles, s);
         if (st != CHY_OK) return st;
-        if (launch_pdl(p->w.pdl, k_wide_sweep, dim3(items), dim3(256), t.M * sizeof(float), s, t, p->mx->dev, d) != cudaSuccess) return CHY_ERR_CUDA;
+        cudaError_t e = cudaSuccess;
+        // rows in tensor memory while its 512 columns hold them (measured above)
+        if (t.M <= 512) {
+            e = ensure_smem((const void *)k_wide_sweep_tm, SwSmem::bytes);
+            if (e == cudaSuccess)
+                e = launch_pdl(p->w.pdl, k_wide_sweep_tm, dim3(std::min(items, p->num_sms)), dim3(256), SwSmem::bytes, s, t, p->mx->dev, d, items);
+        } else {
+            e = launch_pdl(p->w.pdl, k_wide_sweep, dim3(items), dim3(256), t.M * sizeof(float), s, t, p->mx->dev, d);
+        }
+        if (e != cudaSuccess) return CHY_ERR_CUDA;
         st = it == 0   ? (last ? wide_launch(k_wide_up<0, 2>, p, tiles, s, it) : wide_launch(k_wide_up<0, 0>, p, tiles, s, it))
              : it == 1 ? (last ? wide_launch(k_wide_up<1, 2>, p, tiles, s, it) : wide_launch(k_wide_up<1, 1>, p, tiles, s, it))
                        : (last ? wide_launch(k_wide_up<2, 2>, p, tiles, s, it) : wide_launch(k_wide_up<2, 1>, p, tiles, s, it));
