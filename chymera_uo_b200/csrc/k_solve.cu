@@ -99,7 +99,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd_f64(DevTables t, Work w, 
     const int njt = (M + Z::JT - 1) / Z::JT;
     const int items = nb * t.L * njt;   // item = (solve * L + mode) * njt + tile
     const bool even = (J & 1) == 0;
-    const double edge = t.cmmax / t.pig4;
+    // GRAV = 0: the boundary is zero like the sources, and so is its fold
+    const double edge = t.pig4 != 0.0 ? t.cmmax / t.pig4 : 0.0;
     auto load = [&](int it, double *Y) {
         if (it < items) {
             const int q = it / njt, j0 = (it - q * njt) * Z::JT;
