@@ -351,10 +351,10 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     auto al = [](size_t n) { return (n + 31) & ~(size_t)31; };
     const bool blk = precision == CHY_PREC_FP64_BLKTRI;
     const size_t nbvec = blk ? al(blk_vector_doubles(t, max_batch)) : 0;
-    const size_t nbscr = blk ? al(blk_scratch_doubles(t, max_batch, p->num_sms)) : 0;
+    const size_t nbscr = blk ? al(blk_scratch_doubles(t, max_batch, p->num_sms)) : 0, nstat = al(1);
     const size_t per = al(w.sX * max_batch) + al(w.sW * max_batch) +
                        al(w.smom * max_batch) + al(w.ssub * max_batch) + al(w.sscan * max_batch) +
-                       al(w.sphac * max_batch) + al(w.sdiag * max_batch) + nbvec + nbscr;
+                       al(w.sphac * max_batch) + al(w.sdiag * max_batch) + nbvec + nbscr + nstat;
     size_t ext = chy_mixed_work_doubles(p);
     p->work_bytes = (per + ext) * sizeof(double) + 4096;
     ce = cudaMalloc(&p->d_work, p->work_bytes);
@@ -372,6 +372,7 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     w.diag = q; q += al(w.sdiag * max_batch);
     w.bvec = blk ? q : nullptr; q += nbvec;
     w.bscr = blk ? q : nullptr; q += nbscr;
+    w.stat = (int *)q; q += nstat;
     w.coef = nullptr;
     chy_mixed_bind_work(p, q);
     CHY_CUDA(cudaMemset(p->d_work, 0, p->work_bytes));
@@ -383,7 +384,7 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
             return st;
         }
     }
-    CHY_CUDA(cudaMallocHost(&p->h_diag, sizeof(double) * kDiagPart * max_batch));
+    CHY_CUDA(cudaMallocHost(&p->h_diag, sizeof(double) * (kDiagPart * max_batch + 1)));
     *out = p;
     return CHY_OK;
 }
@@ -670,14 +671,27 @@ static int run_batch(chy_plan *p, const BatchPtrs &bp, int nb, cudaStream_t s, b
     return CHY_OK;
 }
 
+static const char kExpired[] = "a bounded wait ran out; what depended on it is NaN in PHI";
+
+cudaError_t chy_internal_read_error(chy_plan *p, int *host_word, cudaStream_t s)
+{
+    const cudaError_t e = cudaMemcpyAsync(host_word, p->w.stat, sizeof(int), cudaMemcpyDeviceToHost, s);
+    return e != cudaSuccess ? e : cudaMemsetAsync(p->w.stat, 0, sizeof(int), s);
+}
+
 static int fetch_diag(chy_plan *p, chy_diag *diag, int nb, int first, cudaStream_t s)
 {
     if (!diag) return CHY_OK;
     CHY_CUDA(cudaMemcpy2DAsync(p->h_diag, sizeof(double) * kDiagPart, p->w.diag, sizeof(double) * p->w.sdiag,
                                sizeof(double) * kDiagPart, nb, cudaMemcpyDeviceToHost, s));
     CHY_CUDA(cudaStreamSynchronize(s));
+    for (int i = 0; i < nb; i++)
+        if (p->h_diag[(size_t)kDiagPart * i + kDiagErr] != 0.0) {
+            CHY_CUDA(cudaMemsetAsync(p->w.stat, 0, sizeof(int), s));
+            return fail(CHY_ERR_TIMEOUT, kExpired);
+        }
     const int st = chy_mixed_collect(p, nb);
-    if (st != CHY_OK) return fail(st, st == CHY_ERR_TIMEOUT ? "mode solve: bounded wait expired" : "mode solve readback");
+    if (st != CHY_OK) return fail(st, "mode solve readback");
     for (int i = 0; i < nb; i++) {
         chy_diag &d = diag[first + i];
         const double *h = p->h_diag + (size_t)kDiagPart * i;
@@ -808,19 +822,13 @@ extern "C" int chy_solve_batch(chy_plan *p, int n, const double *const *rho, dou
     }
     for (int i = 0; i < R; i++)
         if (used[i]) CHY_CUDA(cudaStreamWaitEvent(s, p->ev_out[i], 0));
-    // a bounded wait that expired in any of these mode solves (with diag the
-    // chunks have reported it already)
-    int *err = diag ? nullptr : chy_mixed_host_error_word(p);
-    if (err) {
-        *err = 0;
-        st = chy_mixed_read_error(p, err, s);
-        if (st != CHY_OK) return fail(st, "error word readback");
-    }
+    // a bounded wait that ran out in any of these solves (with diag the chunks
+    // have reported it already)
+    int *err = (int *)(p->h_diag + (size_t)kDiagPart * p->max_batch);
+    *err = 0;
+    if (!diag) CHY_CUDA(chy_internal_read_error(p, err, s));
     CHY_CUDA(cudaStreamSynchronize(s));
-    if (err && *err != 0) {
-        *err = 0;
-        return fail(CHY_ERR_TIMEOUT, "mode solve: a bounded wait expired; the affected modes of PHI are NaN");
-    }
+    if (*err != 0) return fail(CHY_ERR_TIMEOUT, kExpired);
     return CHY_OK;
 }
 
@@ -1226,6 +1234,13 @@ extern "C" int chy_solve_static(chy_plan *p, const double *rho, double *phi, voi
     int nv = 0;
     CHY_CUDA(launch_inverse(t, bp, w, StarDev{}, 1, s, &nv));   // POT3 alone
     p->launches += 1 + 2 + 1 + 3 + nv;
+    return CHY_OK;
+}
+
+extern "C" int chy_dbg_sweep_probe(chy_plan *p, int polls)
+{
+    if (!p || p->precision != CHY_PREC_FP64 || polls < 0) return fail(CHY_ERR_ARG, "probe needs an FP64 plan and polls >= 0");
+    p->w.probe = polls;
     return CHY_OK;
 }
 

@@ -109,6 +109,8 @@ struct Work {
     double *coef;                                    // optional /COEFS/ output (solve 0 only)
     double *bvec, *bscr;                             // BLKTRI-order path (k_blktri.cu)
     bool pdl;                                        // overlap launches (pdl.h)
+    int *stat;                                       // error word: non-zero once a bounded wait has run out
+    int probe;                                       // test hook: polls on a barrier nothing arrives on (0: off)
 };
 
 // ExternalPot (pot/ExternalPot.f:1-80): the star potential added after POT3.
@@ -125,6 +127,7 @@ struct StarDev {
     double mass_bin = 0.0, rbin = 0.0, omega2 = 0.0, rcom = 0.0;
 };
 constexpr int kDiagStar = 4;     // DIAG slots of INDIRECTX, INDIRECTY
+constexpr int kDiagErr = 6;      // DIAG slot of the error word
 constexpr int kDiagPart = 8;     // first DIAG slot of the per-L moments
 
 // SOURCE's potential, pressure and rotation terms (radhydro/source.f:45-81).

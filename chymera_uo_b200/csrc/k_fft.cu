@@ -552,7 +552,10 @@ __global__ void __launch_bounds__(256) k_forward(DevTables t, BatchPtrs bp, Work
             if (jp != kp) xc[(size_t)kp * pl] = (aa - re) * t.sf1;
             if (jp >= 1) xc[(size_t)(n + jp) * pl] = (im + bb) * t.sf1;
             if (jp >= 1 && jp != kp) xc[(size_t)(n + kp) * pl] = (im - bb) * t.sf1;
-            if (!landed) xc[0] = __longlong_as_double(0x7ff8000000000000ll);
+            if (!landed) {
+                xc[0] = __longlong_as_double(0x7ff8000000000000ll);
+                *w.stat = 1;
+            }
         }
     }
 }
@@ -857,6 +860,7 @@ __global__ void __launch_bounds__(256) k_inverse(DevTables t, BatchPtrs bp, Work
         if (threadIdx.x < T::TC) {
             const int c = threadIdx.x;
             A[n * RS + c] = landed ? A[I0 * RS + c] : __longlong_as_double(0x7ff8000000000000ll);
+            if (!landed) *w.stat = 1;
             A[I0 * RS + c] = 0.0;
             A[(I0 + n) * RS + c] = 0.0;
         }
@@ -1078,6 +1082,10 @@ __global__ void __launch_bounds__(32) k_diag(DevTables t, Work w)
     pdl_go();
     pdl_wait();
     const double *phac = w.phac + (size_t)b * w.sphac;
+    // every load before the first store: column 0 = TERM(1)*SUMASS, the inside sum
+    // over all rings, and the error word
+    const double tmass = __ldcg(w.scan + (size_t)b * w.sscan + (size_t)t.nsub * 2 * t.ncol);
+    const int stat = __ldcg(w.stat);
     double err = 0.0;
     int klocat = 0;
     for (int k0 = 2; k0 <= t.K + 1; k0 += 128) {
@@ -1095,10 +1103,10 @@ __global__ void __launch_bounds__(32) k_diag(DevTables t, Work w)
     }
     if (lane != 0) return;
     double *d = w.diag + (size_t)b * w.sdiag;
-    const double *scan = w.scan + (size_t)b * w.sscan;
-    d[0] = scan[(size_t)t.nsub * 2 * t.ncol + 0];   // column 0 = TERM(1)*SUMASS, inside sum over all rings
+    d[0] = tmass;
     d[1] = err;
     d[2] = (double)klocat;
+    d[kDiagErr] = (double)stat;
 }
 
 // ---------------------------------------------------------------------------

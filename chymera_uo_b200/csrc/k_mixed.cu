@@ -113,7 +113,6 @@ struct MixedState {
     MixedDev dev{};
     double *h_corr = nullptr;       // pinned copy of corr
     size_t xbuf_bytes = 0;          // FP64 iterate (two or more corrections)
-    int *h_err = nullptr;           // pinned
     int probe_polls = 0;            // test hook (chy_dbg_mixed_probe)
     WideDev wide{};                 // the multi-kernel pipeline of grids k_mode_mixed does not cover
     bool is_wide = false;
@@ -2624,11 +2623,13 @@ __global__ void __launch_bounds__(256, 1) k_wide_sweep_tm(DevTables t, MixedDev 
             pi += gridDim.x;
         }
     };
-    if (tid == 0)
-        for (int i = 0; i < kSwSlots; ++i) issue();
     int cs = 0;
     uint32_t ph = 0;
     bool ok = true;
+    // test hook: no copy is issued, and the first wait runs out after probe_polls
+    const long long polls = x.probe_polls > 0 ? x.probe_polls : kSpinLimit;
+    if (tid == 0 && x.probe_polls == 0)
+        for (int i = 0; i < kSwSlots; ++i) issue();
     auto next = [&]() {   // this chunk's slot has been read: refill it
         __syncthreads();
         if (tid == 0 && ok) issue();
@@ -2645,7 +2646,8 @@ __global__ void __launch_bounds__(256, 1) k_wide_sweep_tm(DevTables t, MixedDev 
         const float et = __ldg(mul + (size_t)(h - 1) * 128), fu = __ldg(mul + (size_t)h * 128);
         float yp = 0.0f;
         for (int c = 0; c < nc; ++c) {
-            ok = ok && mbar_wait(bar + cs, ph);
+            ok = ok && mbar_wait_n(bar + cs, ph, polls);
+            __syncwarp();   // the warp's tensor-memory accesses are collective
             // the i-th row of the elimination is at i * 128 (upper) or (R-1-i) * 128
             const float *y = ring + cs * 2 * kSwHalf + p, *co = s_tab + c * R;
             const int n = low ? ML - c * R : R;
@@ -2683,7 +2685,8 @@ __global__ void __launch_bounds__(256, 1) k_wide_sweep_tm(DevTables t, MixedDev 
         for (int c = nc - 1; c >= 0; --c) {
             float v[R];
             tm_ld16(tm + c * R, v);
-            ok = ok && mbar_wait(bar + cs, ph);
+            ok = ok && mbar_wait_n(bar + cs, ph, polls);
+            __syncwarp();
             if (!ok) xn = __int_as_float(0x7fc00000);
             const float *e = ring + cs * 2 * kSwHalf + p;
             const int n = low ? min(ML - c * R, R) : R;
@@ -2873,7 +2876,7 @@ void chy_mixed_bind_tables(chy_plan *p, char *dev_base)
     p->mx->dev.sw_piv = p->mx->dev.sw_mul + (size_t)(p->hp.N + 1) * round64(p->hp.J) * 128;
 }
 
-// Per-mode correction sums and the error word; the FP64 iterate of the
+// Per-mode correction sums; the FP64 iterate of the
 // general path (two or more corrections) is allocated by
 // chy_mixed_ensure_iterate when such a count is set.
 static size_t al32(size_t n) { return (n + 31) & ~(size_t)31; }   // doubles, 256-byte pieces
@@ -2889,7 +2892,7 @@ size_t chy_mixed_work_doubles(const chy_plan *p)
 {
     if (p->precision != CHY_PREC_MIXED) return 0;
     const chy::HostPlan &hp = p->hp;
-    size_t n = al32(corr_stride(&hp) * p->max_batch + 8);
+    size_t n = al32(corr_stride(&hp) * p->max_batch);
     if (!mixed_fused(&hp)) {
         const size_t items = (size_t)hp.L * p->max_batch, Jt = (size_t)round64(hp.J);
         n += al32(items * Jt * 128 / 2);                 // W (FP32)
@@ -2908,7 +2911,7 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
     d.scorr = corr_stride(&hp);
     d.xbuf = nullptr;
     d.corr = base;
-    d.err = reinterpret_cast<int *>(d.corr + d.scorr * p->max_batch);
+    d.err = p->w.stat;
     d.ntile = round64(hp.J);
     if (p->precision == CHY_PREC_MIXED && !mixed_fused(&hp)) {
         WideDev &wd = p->mx->wide;
@@ -2917,7 +2920,7 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
         wd.nt = round64(hp.J) / 64;
         wd.sw = (size_t)round64(hp.J) * 128;
         wd.sx = (size_t)hp.NZ * hp.J;
-        double *q = base + al32(d.scorr * p->max_batch + 8);
+        double *q = base + al32(d.scorr * p->max_batch);
         wd.W = reinterpret_cast<float *>(q);
         q += al32(items * wd.sw / 2);
         wd.F = reinterpret_cast<float *>(q);
@@ -2926,7 +2929,6 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
     }
     if (p->precision == CHY_PREC_MIXED) {
         cudaMallocHost(&p->mx->h_corr, sizeof(double) * d.scorr * p->max_batch);
-        cudaMallocHost(&p->mx->h_err, sizeof(int));
         // the residual's right-hand-side tiles: X viewed as max_batch*L*K rows
         // of JX doubles; one item is K consecutive rows
         PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
@@ -2973,6 +2975,8 @@ static int wide_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
 {
     const WideDev &d = p->mx->wide;
     const chy::DevTables &t = p->t;
+    MixedDev x = p->mx->dev;
+    x.probe_polls = p->mx->probe_polls;
     const int nit = std::min(1 + p->refine, 8), items = nb * t.L, tiles = items * d.nt;
     for (int it = 0; it < nit; ++it) {
         const bool last = it == nit - 1;
@@ -2985,7 +2989,7 @@ static int wide_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
         if (t.M <= 512) {
             e = ensure_smem((const void *)k_wide_sweep_tm, SwSmem::bytes);
             if (e == cudaSuccess)
-                e = launch_pdl(p->w.pdl, k_wide_sweep_tm, dim3(std::min(items, p->num_sms)), dim3(256), SwSmem::bytes, s, t, p->mx->dev, d, items);
+                e = launch_pdl(p->w.pdl, k_wide_sweep_tm, dim3(std::min(items, p->num_sms)), dim3(256), SwSmem::bytes, s, t, x, d, items);
         } else {
             e = launch_pdl(p->w.pdl, k_wide_sweep, dim3(items), dim3(256), t.M * sizeof(float), s, t, p->mx->dev, d);
         }
@@ -3075,34 +3079,15 @@ int chy_mixed_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
     return CHY_OK;
 }
 
-// Per-step correction norms ||delta_i|| / ||x_i|| summed over modes, and the
-// device error word.  Called after the stream has been synchronised.
+// Per-step correction norms ||delta_i|| / ||x_i|| summed over modes.  Called after
+// the stream has been synchronised.
 int chy_mixed_collect(chy_plan *p, int nb)
 {
     if (p->precision != CHY_PREC_MIXED || !p->mx) return CHY_OK;
     MixedState &m = *p->mx;
-    if (cudaMemcpy(m.h_err, m.dev.err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return CHY_ERR_CUDA;
-    if (*m.h_err != 0) {
-        cudaMemset(m.dev.err, 0, sizeof(int));
-        return CHY_ERR_TIMEOUT;
-    }
     if (cudaMemcpy(m.h_corr, m.dev.corr, sizeof(double) * m.dev.scorr * nb, cudaMemcpyDeviceToHost) != cudaSuccess)
         return CHY_ERR_CUDA;
     return CHY_OK;
-}
-
-int chy_mixed_read_error(chy_plan *p, int *host_word, cudaStream_t s)
-{
-    if (p->precision != CHY_PREC_MIXED || !p->mx || !host_word) return CHY_OK;
-    if (cudaMemcpyAsync(host_word, p->mx->dev.err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemsetAsync(p->mx->dev.err, 0, sizeof(int), s) != cudaSuccess)
-        return CHY_ERR_CUDA;
-    return CHY_OK;
-}
-
-int *chy_mixed_host_error_word(chy_plan *p)
-{
-    return (p->precision == CHY_PREC_MIXED && p->mx) ? p->mx->h_err : nullptr;
 }
 
 int chy_mixed_last_kernel(const chy_plan *p)
@@ -3166,7 +3151,6 @@ void chy_mixed_release(chy_plan *p)
     if (!p->mx) return;
     cudaFree(p->mx->dev.xbuf);
     cudaFreeHost(p->mx->h_corr);
-    cudaFreeHost(p->mx->h_err);
     delete p->mx;
     p->mx = nullptr;
 }

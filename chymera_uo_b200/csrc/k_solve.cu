@@ -297,10 +297,10 @@ constexpr size_t kTmBytes = kTmSlots * kTmSlotDoubles * 8 + 256 * 8 + kTmSlots *
 
 __device__ __forceinline__ uint32_t tm_sm32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// bounded wait on phase `parity`: false after it ran out
-__device__ __forceinline__ bool tm_bar_wait(uint64_t *bar, uint32_t parity)
+// bounded wait on phase `parity`: false after `limit` polls
+__device__ __forceinline__ bool tm_bar_wait(uint64_t *bar, uint32_t parity, int limit)
 {
-    for (long long i = 0; i < (1ll << 26); ++i) {
+    for (int i = 0; i < limit; ++i) {
         uint32_t done;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(done)
@@ -406,12 +406,14 @@ __global__ void __launch_bounds__(128, 1) k_thomas_tm(DevTables t, Work w, int g
             pg += gridDim.x;
         }
     };
-    if (tid == 0)
-        for (int i = 0; i < kTmSlots; ++i) issue();
-
     int cs = 0;
     uint32_t ph = 0;
     bool ok = true;
+    // test hook: no copy is issued, and the first wait runs out after `probe` polls
+    const int polls = w.probe > 0 ? w.probe : 1 << 26;
+    if (tid == 0 && w.probe == 0)
+        for (int i = 0; i < kTmSlots; ++i) issue();
+
     auto next = [&]() {   // this chunk's slot has been read: refill it
         __syncthreads();
         if (tid == 0 && ok) issue();
@@ -427,7 +429,8 @@ __global__ void __launch_bounds__(128, 1) k_thomas_tm(DevTables t, Work w, int g
         double *Wp = w.W + (size_t)b * w.sW + (size_t)l * t.J * K + p;
         double prev = 0.0;
         for (int c = 0; c < nc; ++c) {
-            ok = ok && tm_bar_wait(bar + cs, ph);
+            ok = ok && tm_bar_wait(bar + cs, ph, polls);
+            __syncwarp();   // the warp's tensor-memory accesses are collective
             const double *y = tsm + cs * kTmSlotDoubles + g * R * K + p, *r = y + R * 128;
             double v[R];
             const int rows = M - c * R;
@@ -451,7 +454,8 @@ __global__ void __launch_bounds__(128, 1) k_thomas_tm(DevTables t, Work w, int g
             double v[R];
             tm_get8(tm + c * 2 * R, v);
             tm_get8(tm + c * 2 * R + 16, v + 8);
-            ok = ok && tm_bar_wait(bar + cs, ph);
+            ok = ok && tm_bar_wait(bar + cs, ph, polls);
+            __syncwarp();
             const double *m = tsm + cs * kTmSlotDoubles + R * 128 + g * R * K + p;
             double *o = Wp + (size_t)c * R * K;
             const int last = M - 1 - c * R;   // the last row's place in its chunk: x as it is
@@ -472,12 +476,14 @@ __global__ void __launch_bounds__(128, 1) k_thomas_tm(DevTables t, Work w, int g
             next();
         }
     }
-    // a wait that ran out: every slot's last copy (bounded) before the memory goes
-    if (tid == 0 && !ok)
-        for (int i = 0; i < kTmSlots; ++i) {
-            const int f = fills / kTmSlots + (i < fills % kTmSlots ? 1 : 0);
-            if (f > 0) tm_bar_wait(bar + i, (uint32_t)(f - 1) & 1u);
-        }
+    if (!ok) {   // a wait that ran out: every slot's last copy (bounded) before the memory goes
+        atomicExch(w.stat, 1);
+        if (tid == 0)
+            for (int i = 0; i < kTmSlots; ++i) {
+                const int f = fills / kTmSlots + (i < fills % kTmSlots ? 1 : 0);
+                if (f > 0) tm_bar_wait(bar + i, (uint32_t)(f - 1) & 1u, polls);
+            }
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (tid < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(*slot));

@@ -47,7 +47,7 @@ struct chy_plan {
     cudaStream_t s_h2d = nullptr, s_d2h = nullptr;
     cudaEvent_t ev_start = nullptr;
     cudaEvent_t ev_in[kStageSlots] = {}, ev_done[kStageSlots] = {}, ev_out[kStageSlots] = {};
-    double *h_diag = nullptr;   // pinned
+    double *h_diag = nullptr;   // pinned; the last double holds a copy of the error word
     double *coef_host = nullptr;   // /COEFS/ host destination (chy_plan_set_coef_host)
     double *coef_dev = nullptr;    // device COEF buffer owned by the plan
     size_t coef_bytes = 0;
@@ -119,6 +119,11 @@ cudaError_t chy_internal_rim_in(double *dev, const double *src, int J, int K, in
 // Sets the calling thread's chy_last_error message; returns code (api.cu).
 int chy_internal_fail(int code, const char *msg);
 
+// Enqueues on s a copy of the plan's device error word into *host_word (pinned)
+// and its reset; the word is non-zero after the stream is synchronised if a
+// bounded wait of an earlier solve ran out (api.cu).
+cudaError_t chy_internal_read_error(chy_plan *p, int *host_word, cudaStream_t s);
+
 // One launch sequence over nb device-pointer solves (api.cu).
 int chy_internal_run_batch(chy_plan *p, const chy::BatchPtrs &bp, int nb, cudaStream_t s);
 
@@ -138,16 +143,9 @@ size_t chy_mixed_work_doubles(const chy_plan *p);
 void chy_mixed_bind_work(chy_plan *p, double *base);
 // Solves the modes of nb solves in place in X; reports its launch count.
 int chy_mixed_solve(chy_plan *p, int nb, cudaStream_t s, int *launches);
-// After a stream sync: reads the device error word and the per-mode
-// correction norms; CHY_ERR_TIMEOUT if a bounded wait expired.
+// After a stream sync: reads the per-mode correction norms.
 int chy_mixed_collect(chy_plan *p, int nb);
 void chy_mixed_fill_diag(const chy_plan *p, int slot, chy_diag *d);
-// Enqueues on s a copy of the device error word into *host_word (pinned)
-// and its reset; the word is non-zero after the stream is synchronised if a
-// bounded wait of an earlier mode solve expired.  No-op for other paths.
-int chy_mixed_read_error(chy_plan *p, int *host_word, cudaStream_t s);
-// The plan's own pinned error word (mixed plans), else null.
-int *chy_mixed_host_error_word(chy_plan *p);
 // Test hook behind chy_dbg_mixed_probe.
 // The kernel of the plan's last mixed mode solve: 0 none / not mixed, 1 k_mode_mixed,
 // 2 k_mode_pair, 3 the wide pipeline.

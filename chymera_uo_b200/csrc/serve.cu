@@ -58,7 +58,7 @@ struct Request {
 };
 
 // One batch in flight: its requests, the events that order its copies in,
-// solve and copies out, and the pinned word its mode solve's error word is
+// solve and copies out, and the pinned word its plan's error word is
 // read back into.
 struct Slot {
     std::vector<Request *> batch;
@@ -312,11 +312,10 @@ int chy_server::launch(SizeClass &c, Lane &ln, Slot &sl)
             return CHY_ERR_CUDA;
     int st = chy_internal_run_batch(ln.plan, bp, nb, ln.stream);
     if (st != CHY_OK) return st;
-    // the mode solve's error word, read back with the batch into the slot's own
-    // word (checked at retirement; no-op for other precisions)
+    // the plan's error word, read back with the batch into the slot's own word
+    // (checked at retirement)
     *sl.err = 0;
-    st = chy_mixed_read_error(ln.plan, sl.err, ln.stream);
-    if (st != CHY_OK) return st;
+    if (chy_internal_read_error(ln.plan, sl.err, ln.stream) != cudaSuccess) return CHY_ERR_CUDA;
     if (cudaEventRecord(sl.solved, ln.stream) != cudaSuccess ||
         cudaStreamWaitEvent(ln.s_out, sl.solved, 0) != cudaSuccess)
         return CHY_ERR_CUDA;

@@ -50,8 +50,14 @@ int chy_dbg_umma(chy_plan *p, int which, const float *Bm_dev, float *D_dev, int 
  * the plan's later mode solves first waits `polls` polls on a barrier that
  * nothing arrives on, before it issues any copy or product; the wait runs
  * out, the CTA poisons its modes with NaN, sets the device error word and
- * exits, and the solve reports CHY_ERR_TIMEOUT.  0 switches it off. */
+ * exits, and the solve reports CHY_ERR_TIMEOUT.  On the wide pipeline the sweeps
+ * in tensor memory (JMAX <= 513) run out so.  0 switches it off. */
 int chy_dbg_mixed_probe(chy_plan *p, int polls);
+
+/* The same for the radial sweeps in tensor memory of a CHY_PREC_FP64 plan: no
+ * copy is issued and each CTA's first wait runs out after `polls` polls; its modes
+ * become NaN and the solve reports CHY_ERR_TIMEOUT.  0 switches it off. */
+int chy_dbg_sweep_probe(chy_plan *p, int polls);
 
 /* The kernel that ran the plan's last mixed mode solve: 1 k_mode_mixed (one
  * CTA per mode), 2 k_mode_pair (CTA pairs), 3 the wide pipeline, 0 none yet or
