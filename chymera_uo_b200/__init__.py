@@ -146,6 +146,8 @@ def lib():
         L.chy_dbg_mixed_probe.restype = i
         L.chy_dbg_sweep_probe.argtypes = [vp, i]
         L.chy_dbg_sweep_probe.restype = i
+        L.chy_dbg_blk_redone.argtypes = []
+        L.chy_dbg_blk_redone.restype = ll
         L.chy_dbg_mixed_kernel.argtypes = [vp]
         L.chy_dbg_mixed_kernel.restype = i
         L.chy_dbg_blktri.argtypes = [C.POINTER(ChyGrid), i, C.POINTER(C.c_double)]

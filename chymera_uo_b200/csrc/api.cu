@@ -1237,6 +1237,13 @@ extern "C" int chy_solve_static(chy_plan *p, const double *rho, double *phi, voi
     return CHY_OK;
 }
 
+extern "C" long long chy_dbg_blk_redone(void)
+{
+    unsigned n = 0;
+    const cudaError_t e = blk_redone(&n);
+    return e == cudaSuccess ? (long long)n : -cuda_fail(e, "chy_dbg_blk_redone");
+}
+
 extern "C" int chy_dbg_sweep_probe(chy_plan *p, int polls)
 {
     if (!p || p->precision != CHY_PREC_FP64 || polls < 0) return fail(CHY_ERR_ARG, "probe needs an FP64 plan and polls >= 0");

@@ -176,6 +176,8 @@ bool blk_schedule_valid(int nw, int ctas_per_sm);
 size_t blk_table_doubles(int M, int L, int nroots);
 int blk_table_blocks(int L);
 cudaError_t launch_blk_table(const DevTables &t, int nroots, double *tab, int *bad, cudaStream_t s);
+// Test hook: its passes so far that the table did not settle (waits for the device).
+cudaError_t blk_redone(unsigned *n);
 // Its work-space sizes in doubles: BVEC for nb solves, BSCR for a plan of max_batch.
 size_t blk_vector_doubles(const DevTables &t, int nb);
 size_t blk_scratch_doubles(const DevTables &t, int max_batch, int num_sms);

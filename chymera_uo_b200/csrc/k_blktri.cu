@@ -373,11 +373,16 @@ struct BlkWarp {
     uint32_t cm;      // CM, [Mp] doubles, the same for every lane
 };
 
+// Passes formed again with divisions on this device so far, for the tests (as a
+// plan's word it would take a register of every pass: 1% of a solve).
+__device__ unsigned g_blk_redone;
+
 // The chunk of rows i0 .. i0-7 again, with IEEE divisions: one whose quotients
 // the tabulated reciprocals did not settle.  dd: the table's D.
 __device__ __noinline__ double blk_elim_div(uint32_t y, uint32_t cm, const double *bm, const double *dd, double rt, int m,
                                             int i0, double wn, double *o)
 {
+    if (i0 < 8 && (threadIdx.x & 31) == 0) atomicAdd(&g_blk_redone, 1u);   // the pass's last chunk
 #pragma unroll 1
     for (int u = 0; u < 8; ++u) {
         const int i = i0 - u;
@@ -538,6 +543,9 @@ __device__ __noinline__ void blk_prdct_tab(const BlkProg &pg, const BlkStep *__r
             }
         }
         if (__any_sync(0xffffffffu, bad)) {
+            // the rows stored above go to the same columns as these: no order among
+            // stores in flight
+            if constexpr (TM) blk_tm_wait_st();
             wn = 0.0;
 #pragma unroll 1
             for (int c = 0; c < nc; ++c) {
@@ -545,6 +553,7 @@ __device__ __noinline__ void blk_prdct_tab(const BlkProg &pg, const BlkStep *__r
                 wn = blk_elim_div(bw.y, bw.cm, bm, tq + dofs, sp.rt, m, mp - 1 - 8 * c, wn, div);
 #pragma unroll
                 for (int u = 0; u < 8; ++u) up[u] = div[7 - u];
+                __syncwarp();   // the store is the warp's
                 keep(c, up);
             }
         }
@@ -851,5 +860,7 @@ cudaError_t launch_solve_blk(const DevTables &t, const Work &w, int nb, int num_
     if (launches) *launches = 3;
     return launch_pdl(w.pdl, k_blk_scatter, dim3(ngroups, t.NZ, rtiles), dim3(256), 0, s, t, w, nb);
 }
+
+cudaError_t blk_redone(unsigned *n) { return cudaMemcpyFromSymbol(n, g_blk_redone, sizeof *n); }
 
 }  // namespace chy

@@ -59,6 +59,11 @@ int chy_dbg_mixed_probe(chy_plan *p, int polls);
  * become NaN and the solve reports CHY_ERR_TIMEOUT.  0 switches it off. */
 int chy_dbg_sweep_probe(chy_plan *p, int polls);
 
+/* PRDCT passes of BLKTRI-order solves on the current device so far that the
+ * tabulated pivots did not settle and that were formed again with divisions;
+ * waits for the device. */
+long long chy_dbg_blk_redone(void);
+
 /* The kernel that ran the plan's last mixed mode solve: 1 k_mode_mixed (one
  * CTA per mode), 2 k_mode_pair (CTA pairs), 3 the wide pipeline, 0 none yet or
  * not a CHY_PREC_MIXED plan; -CHY_ERR_ARG for a null plan. */
