@@ -506,7 +506,6 @@ __global__ void __launch_bounds__(256, 1) k_mode_mixed(DevTables t, Work w, Mixe
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_cv + 1);
     int *s_flag = reinterpret_cast<int *>(tmem_slot + 1);
 
-    pdl_go();
     // ---- setup: tensor memory (all 512 columns), barriers, m-independent tables
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
@@ -1220,6 +1219,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_mixed(DevTables t, Work w, Mixe
     }
     // drain copies and products still in flight (bounded), then release
     // tensor memory
+    pdl_go();
     if (a_inflight) mbar_wait(bar_a, ph_a);
     for (int sl = 0; sl < kRingSlots; ++sl)
         if (ring_pend & (1u << sl)) mbar_wait(bar_ring + sl, (ring_ph >> sl) & 1u);
@@ -2104,7 +2104,6 @@ __global__ void __launch_bounds__(256, 2) k_wide_down(DevTables t, Work w, Mixed
 {
     extern __shared__ __align__(1024) uint8_t sm[];
     WideCta c;
-    pdl_go();
     wide_setup(c, sm, t, x);
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, M = t.M, NZ = t.NZ, J = t.JX, k0 = 16 * warp;
@@ -2165,6 +2164,7 @@ __global__ void __launch_bounds__(256, 2) k_wide_down(DevTables t, Work w, Mixed
         const double xl2 = 2.0 * (t.xlamm[m] - 1.0);
         const double *Xl = w.X + (size_t)item * t.K * J;
         const bool more = tile + (int)gridDim.x < tiles;
+        if (!more) pdl_go();
         if (more) {   // the next tile: KMAX rows of 512 bytes of X, 256 of F
             const int nt = tile + gridDim.x, ni = nt / d.nt, nj = (nt - ni * d.nt) * kWideT;
             for (int i = threadIdx.x; i < 4 * t.K; i += 256)
@@ -2339,7 +2339,6 @@ __global__ void __launch_bounds__(256, 2) k_wide_up(DevTables t, Work w, MixedDe
 {
     extern __shared__ __align__(1024) uint8_t sm[];
     WideCta c;
-    pdl_go();
     wide_setup(c, sm, t, x);
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, M = t.M, NZ = t.NZ;
@@ -2348,6 +2347,7 @@ __global__ void __launch_bounds__(256, 2) k_wide_up(DevTables t, Work w, MixedDe
         const int item = tile / d.nt, j0 = (tile - item * d.nt) * kWideT;
         // rows j0 + warp + 8 i, values p = 4 lane .. 4 lane + 3
         const float *src = d.W + (size_t)item * d.sw + (size_t)(j0 + warp) * 128 + 4 * lane;
+        if (tile + (int)gridDim.x >= tiles) pdl_go();
         if (tile + (int)gridDim.x < tiles) {   // the next tile: 32 KB of W, 256-byte rows of the iterate
             const int nt = tile + gridDim.x, ni = nt / d.nt, nj = (nt - ni * d.nt) * kWideT;
             if (threadIdx.x == 0) l2_prefetch_bulk(d.W + (size_t)ni * d.sw + (size_t)nj * 128, kWideT * 512);

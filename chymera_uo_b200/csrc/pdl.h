@@ -10,6 +10,19 @@
 // constants, also where it then has nothing to do, so that a kernel's completion
 // implies that of all kernels before it.
 //
+// Tensor memory is allocated by waiting until it is free, so a kernel that waits
+// in pdl_wait() with columns in hand must not be able to reach an SM before an
+// earlier kernel has its own there.  A kernel that allocates before pdl_wait()
+// therefore hands over (pdl_go()) only after its allocation; one that allocates
+// after it (k_thomas_tm, k_wide_sweep_tm) fills its SM's shared memory, so that no
+// CTA with columns fits beside it.  The mode solves hand over late, k_mode_mixed at
+// its end and the wide products with their last tile: CTAs that wait through a
+// long kernel take its registers, L1 and issue slots.  Solves one after the other in
+// a graph, hand-over at the start / so (us): mixed 64x32x64 55.4 / 47.6, 256x128x256
+// 246.0 / 241.6, 65x32x64 83.7 / 77.5, 512x64x256 464 / 449; one solve waited for:
+// 71.5 / 70.1, 265.1 / 262.9, 93.9 / 91.0, 496 / 479 (the wide products at their end:
+// 447, but 495 waited for).
+//
 // Waiting CTAs hold registers and shared memory, and a kernel that starts beside
 // one with much shared memory keeps that one's small L1.  So launches overlap
 // (Work::pdl) in a solve that has the device to itself and is short: up to
