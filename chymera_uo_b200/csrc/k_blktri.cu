@@ -644,7 +644,10 @@ __device__ __forceinline__ void blk_group_sync(int ctas)
 // another CTA may have written are read past L1.  Dynamic shared memory: CM
 // (Mp doubles), then per warp ring, right-hand side column and, without TM, the
 // column of partial solutions.  One CTA per SM (the launch asks for over half of
-// the shared memory), so tensor memory is never waited for.
+// the shared memory), so tensor memory is never waited for.  Hands over at its end:
+// the next solve's clusters, resident and waiting through this one, held the SMs
+// that a second stream's solve needs (two plans on two streams, 128x64x128 4.04 ->
+// 2.07 ms a pair, 256x128x256 17.5 -> 12.4; one solve of 64x32x64 567 -> 561 us).
 template <bool TM>
 __global__ void __launch_bounds__(128, 1) k_blk_solve_tab(DevTables t, Work w, int ngroups, int ctas)
 {
@@ -672,7 +675,6 @@ __global__ void __launch_bounds__(128, 1) k_blk_solve_tab(DevTables t, Work w, i
     }
     __syncthreads();
     if constexpr (TM) bw.tm = tm_base + ((uint32_t)(warp * 32) << 16);
-    pdl_go();
     pdl_wait();
     const size_t rstride = (size_t)d.ntab * 3 * col;
     const int worker = rank + ctas * warp, workers = ctas * nw;
@@ -739,6 +741,7 @@ __global__ void __launch_bounds__(128, 1) k_blk_solve_tab(DevTables t, Work w, i
             blk_group_sync(ctas);
         }
     }
+    pdl_go();
     if constexpr (TM) {
         __syncthreads();
         if (warp == 0) {
