@@ -84,7 +84,6 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd_f64(DevTables t, Work w, 
     extern __shared__ __align__(16) double smem[];   // [3][KP][LDY]
     const int NZ = t.NZ, M = t.M, J = t.J, K = t.K, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wp = warp % Z::NWP, wj = warp / Z::NWP;
-    pdl_go();
     double u[Z::KS];
 #pragma unroll
     for (int s = 0; s < Z::KS; ++s) {
@@ -125,6 +124,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd_f64(DevTables t, Work w, 
     load(it, smem);
     load(it + (int)gridDim.x, smem + Z::kFwdBuf);
     for (int buf = 0; it < items; it += gridDim.x, buf = buf == 2 ? 0 : buf + 1) {
+        if (it + (int)gridDim.x >= items) pdl_go();
         double *Yt = smem + buf * Z::kFwdBuf;
         z_wait<1>();
         __syncthreads();
@@ -202,7 +202,6 @@ __global__ void __launch_bounds__(128) k_thomas_f64(DevTables t, Work w)
     const int M = t.M, K = KC ? KC : t.K, p = threadIdx.x % K, b = blockIdx.y;
     const int l = blockIdx.x * (blockDim.x / K) + threadIdx.x / K;
     extern __shared__ double am[];
-    pdl_go();
     for (int j = threadIdx.x; j < M; j += blockDim.x) am[j] = t.am[j];
     __syncthreads();
     pdl_wait();
@@ -279,6 +278,7 @@ __global__ void __launch_bounds__(128) k_thomas_f64(DevTables t, Work w)
         if (c + 2 < nf) load_up(ya, ta);
         if (c + 1 < nf) up(yb, tb);
     }
+    pdl_go();
 }
 
 // The same sweeps with the eliminated rows on chip, for grids of at most 256 rows
@@ -599,8 +599,13 @@ static cudaError_t solve_fp64(const DevTables &t, const Work &w, int nb, int num
             if (e == cudaSuccess)
                 e = launch_pdl(w.pdl, k_thomas_tm<KP>, dim3(groups < num_sms ? groups : num_sms), dim3(128), kTmBytes, s, t, w, groups);
         }
+    // k_thomas_f64 never starts early, and hands over at its end: beside a product's
+    // 200 KB of shared memory its streaming loads have next to no L1.  Solves one
+    // after the other in a graph, both overlapped / so (us): 512x32x64 197 / 91,
+    // 300x128x64 217 / 176, 512x64x256 452 / 296, 128x64x128 x4 175 / 154, 64x32x64
+    // x32 219 / 214; with only its own early start left 91, 199, 416, 175, 218.
     if (!on_chip)
-        e = launch_pdl(w.pdl, sweep, dim3((t.L + mpb - 1) / mpb, nb), dim3(128), (size_t)t.M * sizeof(double), s, t, w);
+        e = launch_pdl(false, sweep, dim3((t.L + mpb - 1) / mpb, nb), dim3(128), (size_t)t.M * sizeof(double), s, t, w);
     if (e != cudaSuccess) return e;
     return launch_pdl(w.pdl, k_zinv_f64<KP, MT>, dim3(grid), dim3(kZThreads), Z::kInvBytes, s, t, w, nb);
 }
