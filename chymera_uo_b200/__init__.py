@@ -113,6 +113,12 @@ def lib():
         L.chy_grid_defaults.argtypes = [C.POINTER(ChyGrid), i, i, i]
         L.chy_plan_create.argtypes = [C.POINTER(ChyGrid), i, i, C.POINTER(vp)]
         L.chy_plan_create.restype = i
+        L.chy_plan_create_limited.argtypes = [C.POINTER(ChyGrid), i, i, ll, C.POINTER(vp)]
+        L.chy_plan_create_limited.restype = i
+        L.chy_plan_set_pivot_table.argtypes = [vp, ll]
+        L.chy_plan_set_pivot_table.restype = i
+        L.chy_plan_pivot_table_bytes.argtypes = [vp]
+        L.chy_plan_pivot_table_bytes.restype = ll
         L.chy_plan_destroy.argtypes = [vp]
         L.chy_solve.argtypes = [vp, vp, vp, C.POINTER(ChyDiag), i, vp]
         L.chy_solve.restype = i
@@ -233,15 +239,17 @@ def precision_code(precision: str) -> int:
 
 
 class Plan:
-    """Per-grid tables + device work space for up to ``max_batch`` solves."""
+    """Per-grid tables + device work space for up to ``max_batch`` solves.
+    ``pivot_table_max``: most bytes of a "blktri" plan's pivot table (0: none,
+    -1: the library's rule, see ``chy_plan_create_limited``)."""
 
-    def __init__(self, g: ChyGrid, precision: str = "fp64", max_batch: int = 1):
+    def __init__(self, g: ChyGrid, precision: str = "fp64", max_batch: int = 1, pivot_table_max: int = -1):
         self.grid = g
         self.precision = precision
         self.shape = (g.jmax + 2, g.kmax + 2, g.lmax)
         p = C.c_void_p()
         prec = precision_code(precision)
-        _check(lib().chy_plan_create(C.byref(g), prec, max_batch, C.byref(p)))
+        _check(lib().chy_plan_create_limited(C.byref(g), prec, max_batch, pivot_table_max, C.byref(p)))
         self._p = p
         self.max_batch = max_batch
 
@@ -267,6 +275,14 @@ class Plan:
     @property
     def launches(self) -> int:
         return lib().chy_plan_launch_count(self._p)
+
+    @property
+    def pivot_table_bytes(self) -> int:
+        return lib().chy_plan_pivot_table_bytes(self._p)
+
+    def set_pivot_table(self, max_bytes: int):
+        """Makes or gives back a "blktri" plan's pivot table (chy_plan_set_pivot_table)."""
+        _check(lib().chy_plan_set_pivot_table(self._p, max_bytes))
 
     def set_refine(self, corrections: int):
         _check(lib().chy_plan_set_refine(self._p, corrections))

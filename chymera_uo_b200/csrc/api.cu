@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -92,30 +93,48 @@ static int check_device(const chy_plan *p)
     return CHY_OK;
 }
 
-// The BLKTRI-order path's pivot table.  It only saves time, so it is left out
-// where it would take more than kBlkTableMax bytes or leave less than half of
-// the device's memory free, or where a pivot is out of the range its quotients
-// need.
+// The BLKTRI-order path's pivot table only saves time.  By default (max_bytes < 0) a
+// plan has one where it takes at most kBlkTableMax bytes, the tables of this process
+// on the device together stay below a sixteenth of its memory, and as much is left
+// free after it: many plans, and whatever else the caller allocates, still fit.  A
+// caller's own limit stands instead of all three; then a table that cannot be
+// allocated is an error.  No plan has one where a pivot is out of the range its
+// quotients need.
 static constexpr size_t kBlkTableMax = (size_t)2 << 30;
-static int make_blk_table(chy_plan *p, int nroots)
+static std::atomic<size_t> g_blktab_bytes[64];   // per device
+
+static int make_blk_table(chy_plan *p, long long max_bytes)
 {
-    const size_t n = blk_table_doubles(p->t.M, p->t.L, nroots), bytes = n * sizeof(double) + 256;
+    const size_t n = blk_table_doubles(p->t.M, p->t.L, p->blk_nroots), bytes = n * sizeof(double) + 256;
+    const bool rule = max_bytes < 0;
+    if (n == 0 || p->blk_untabled || bytes > (rule ? kBlkTableMax : (size_t)max_bytes)) return CHY_OK;
+    std::atomic<size_t> &all = g_blktab_bytes[p->device & 63];
     size_t free_b = 0, total = 0;
-    if (n == 0 || bytes > kBlkTableMax) return CHY_OK;
     CHY_CUDA(cudaMemGetInfo(&free_b, &total));
-    if (free_b < bytes + total / 2) return CHY_OK;
-    if (cudaMalloc(&p->d_blktab, bytes) != cudaSuccess) {
+    const size_t sum = all.fetch_add(bytes) + bytes;
+    double *tab = nullptr;
+    bool have = !rule || (sum <= total / 16 && free_b >= bytes + total / 16);
+    const bool asked = have;
+    if (have && cudaMalloc(&tab, bytes) != cudaSuccess) {
         cudaGetLastError();
-        p->d_blktab = nullptr;
-        return CHY_OK;
+        have = false;
     }
-    int *bad = (int *)(p->d_blktab + n), h_bad = 0;
-    CHY_CUDA(cudaMemset(bad, 0, sizeof(int)));
-    CHY_CUDA(launch_blk_table(p->t, nroots, p->d_blktab, bad, cudaStreamLegacy));
-    CHY_CUDA(cudaMemcpy(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost));
+    if (!have) {
+        all.fetch_sub(bytes);
+        return rule || !asked ? CHY_OK : fail(CHY_ERR_NOMEM, "pivot table");
+    }
+    p->d_blktab = tab;
     p->blktab_bytes = bytes;
-    p->t.blk.tab = p->d_blktab;
-    if (h_bad) chy_internal_drop_blk_table(p);
+    int *bad = (int *)(tab + n), h_bad = 0;
+    CHY_CUDA(cudaMemset(bad, 0, sizeof(int)));
+    CHY_CUDA(launch_blk_table(p->t, p->blk_nroots, tab, bad, cudaStreamLegacy));
+    CHY_CUDA(cudaMemcpy(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost));
+    if (h_bad) {
+        p->blk_untabled = true;
+        chy_internal_drop_blk_table(p);
+    } else {
+        p->t.blk.tab = tab;
+    }
     return CHY_OK;
 }
 
@@ -170,7 +189,7 @@ void chy_plan_destroy(chy_plan *p)
             if (e) cudaEventDestroy(e);
     cudaFree(p->d_tables);
     cudaFree(p->d_work);
-    cudaFree(p->d_blktab);
+    chy_internal_drop_blk_table(p);
     cudaFree(p->stage);
     cudaFree(p->coef_dev);
     for (int i = 0; i < chy_plan::kStageSlots; i++) {
@@ -187,6 +206,11 @@ void chy_plan_destroy(chy_plan *p)
 }
 
 int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **out)
+{
+    return chy_plan_create_limited(g, precision, max_batch, -1, out);
+}
+
+int chy_plan_create_limited(const chy_grid *g, int precision, int max_batch, long long pivot_table_max, chy_plan **out)
 {
     if (!g || !out || max_batch < 1) return fail(CHY_ERR_ARG, "null descriptor/output or max_batch < 1");
     if (precision != CHY_PREC_FP64 && precision != CHY_PREC_MIXED && precision != CHY_PREC_FP64_BLKTRI)
@@ -243,7 +267,6 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     const size_t o_zw = pk.vec(hp.zw), o_tc = pk.vec(hp.term_col);
     size_t o_U = pk.vec(hp.U), o_V = pk.vec(hp.V), o_lam = pk.vec(hp.lam);
     std::vector<double> roots;   // distinct shifts of the schedule
-    bool blk_none = false;
     size_t o_brt = 0;
     size_t o_bst = 0, o_bpg = 0, o_btk = 0, o_bsg = 0, o_bmt = 0;
     if (precision == CHY_PREC_FP64_BLKTRI) {
@@ -252,8 +275,9 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
             const auto at = index.emplace(st.rt, (int)roots.size());
             if (at.second) roots.push_back(st.rt);
             st.pad = at.first->second;
-            blk_none |= st.post == BLK_NONE;
+            p->blk_untabled |= st.post == BLK_NONE;
         }
+        p->blk_nroots = (int)roots.size();
         o_brt = pk.vec(roots);
         o_bst = pk.vec(bs.steps);
         o_bpg = pk.vec(bs.progs);
@@ -377,8 +401,8 @@ int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **
     chy_mixed_bind_work(p, q);
     CHY_CUDA(cudaMemset(p->d_work, 0, p->work_bytes));
     p->nvol = (size_t)(hp.J + 2) * (hp.K + 2) * hp.L;
-    if (blk && !blk_none) {
-        st = make_blk_table(p, (int)roots.size());
+    if (blk) {
+        st = make_blk_table(p, pivot_table_max);
         if (st != CHY_OK) {
             chy_plan_destroy(p);
             return st;
@@ -565,6 +589,17 @@ long long chy_plan_device_bytes(const chy_plan *p)
     if (!p) return 0;
     return (long long)(p->table_bytes + p->blktab_bytes + p->work_bytes + p->stage_bytes + p->coef_bytes + chy_mixed_iterate_bytes(p));
 }
+
+int chy_plan_set_pivot_table(chy_plan *p, long long max_bytes)
+{
+    if (!p || p->precision != CHY_PREC_FP64_BLKTRI) return fail(CHY_ERR_ARG, "pivot tables belong to BLKTRI-order plans");
+    const int st = check_device(p);
+    if (st != CHY_OK) return st;
+    if (max_bytes >= 0 && p->blktab_bytes > (size_t)max_bytes) chy_internal_drop_blk_table(p);
+    return p->d_blktab ? CHY_OK : make_blk_table(p, max_bytes);
+}
+
+long long chy_plan_pivot_table_bytes(const chy_plan *p) { return p ? (long long)p->blktab_bytes : 0; }
 
 long long chy_plan_bytes_per_solve(const chy_plan *p)
 {
@@ -1069,7 +1104,9 @@ extern "C" int chy_autotune_multi(int n, chy_plan *const *plans, const double *c
 size_t chy_internal_drop_blk_table(chy_plan *p)
 {
     const size_t bytes = p->blktab_bytes;
+    if (!p->d_blktab) return 0;
     cudaFree(p->d_blktab);   // waits for the launches that read it
+    g_blktab_bytes[p->device & 63].fetch_sub(bytes);
     p->d_blktab = nullptr;
     p->blktab_bytes = 0;
     p->t.blk.tab = nullptr;

@@ -33,6 +33,8 @@ struct chy_plan {
     size_t table_bytes = 0;
     double *d_blktab = nullptr;    // BLKTRI order: pivot table (null: passes divide)
     size_t blktab_bytes = 0;
+    int blk_nroots = 0;            // distinct shifts of its schedule
+    bool blk_untabled = false;     // its passes or pivots admit no table
     char *d_work = nullptr;
     size_t work_bytes = 0;
     chy::Work w{};

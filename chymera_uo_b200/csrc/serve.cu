@@ -42,6 +42,7 @@ namespace {
 using Clock = std::chrono::steady_clock;
 constexpr int kLanes = 2;
 constexpr int kLaneDepth = 2;   // batches in flight per lane
+constexpr size_t kTableMax = (size_t)2 << 30;   // a plan's pivot table
 
 struct Request {
     long long id = 0;
@@ -231,7 +232,7 @@ int chy_server::make_class(Request *rq, SizeClass **out)
     for (int i = 0; i < kLanes; i++) {
         Lane &ln = c->lanes[i];
         int prec = precision;
-        int st = chy_plan_create(&g, prec, max_batch, &ln.plan);
+        int st = chy_plan_create_limited(&g, prec, max_batch, 0, &ln.plan);   // pivot tables below
         if (st == CHY_ERR_UNSUPPORTED && prec == CHY_PREC_MIXED) {   // grids the mixed path does not cover
             prec = CHY_PREC_FP64;
             st = chy_plan_create(&g, prec, max_batch, &ln.plan);
@@ -249,13 +250,12 @@ int chy_server::make_class(Request *rq, SizeClass **out)
         }
     }
     c->last_use = Clock::now();
-    // over budget: first the BLKTRI pivot tables go, which only save time (this
-    // thread is the only one that launches with these plans)
+    // over budget: first the other classes' BLKTRI pivot tables go, which only save
+    // time (this thread is the only one that launches with these plans)
     auto drop_tables = [&](SizeClass &o) {
         for (Lane &ln : o.lanes)
             if (plan_bytes > budget - arena.size) plan_bytes -= chy_internal_drop_blk_table(ln.plan);
     };
-    drop_tables(*c);
     for (auto &kv : classes) drop_tables(*kv.second);
     // plans count against the budget left after the arena: drop idle classes
     // (least recently used first) to make room, else give up on this grid
@@ -280,6 +280,12 @@ int chy_server::make_class(Request *rq, SizeClass **out)
             lane_free(ln);
         }
         return CHY_ERR_CAPACITY;
+    }
+    // what the budget leaves goes to this class's tables
+    for (Lane &ln : c->lanes) {
+        const size_t left = budget - arena.size - plan_bytes;
+        if (precision != CHY_PREC_FP64_BLKTRI || chy_plan_set_pivot_table(ln.plan, (long long)std::min(left, kTableMax)) != CHY_OK) continue;
+        plan_bytes += (size_t)chy_plan_pivot_table_bytes(ln.plan);
     }
     *out = c.get();
     classes[c->key] = std::move(c);

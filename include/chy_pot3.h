@@ -107,6 +107,25 @@ void chy_grid_defaults(chy_grid *g, int jmax, int kmax, int lmax);
 int chy_plan_create(const chy_grid *g, int precision, int max_batch, chy_plan **out);
 void chy_plan_destroy(chy_plan *p);
 
+/* A BLKTRI-order plan may also keep a table of the pivots of every distinct shift
+ * of its cyclic reduction, which spares its passes their divisions (several times
+ * faster, the same bits): 1 MB a shift at 256 x 128 x 256, some hundred MB in all.
+ * chy_plan_create makes one of at most 2 GiB as long as the tables of all plans of
+ * the process on the device take no more than 1/16 of its memory and 1/16 stays
+ * free.  chy_plan_create_limited takes the limit from the caller instead:
+ * pivot_table_max = 0 makes none, -1 is chy_plan_create's rule, else a table of at
+ * most that many bytes is made (CHY_ERR_NOMEM if it cannot be allocated).  The limit
+ * does not matter to plans of other precisions. */
+int chy_plan_create_limited(const chy_grid *g, int precision, int max_batch, long long pivot_table_max, chy_plan **out);
+/* The same for an existing BLKTRI-order plan (CHY_ERR_ARG for others): a table above
+ * the limit is given back once the device has finished with it, a missing one that
+ * the limit allows is made.  CUDA graphs captured with the plan before refer to the
+ * table as it was: capture them again. */
+int chy_plan_set_pivot_table(chy_plan *p, long long max_bytes);
+/* Device bytes of the plan's pivot table, 0 without one (part of
+ * chy_plan_device_bytes). */
+long long chy_plan_pivot_table_bytes(const chy_plan *p);
+
 /* Every solve entry point needs the device that was current at
  * chy_plan_create to be current when it is called; otherwise it returns
  * CHY_ERR_ARG. */
