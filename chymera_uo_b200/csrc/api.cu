@@ -1017,13 +1017,15 @@ extern "C" int chy_autotune_multi(int n, chy_plan *const *plans, const double *c
     if (n <= 0 || !plans || !rho || !phi) return fail(CHY_ERR_ARG, "empty or null request set");
     if (repeats < 1) repeats = 3;
     std::vector<chy_plan *> uniq;
-    bool any_mixed = false, any_blk = false;
+    bool any_mixed = false, any_blk = false;   // any_blk: with a stage schedule to choose
     int max_batch = 1;
     for (int i = 0; i < n; i++) {
         if (!plans[i]) return fail(CHY_ERR_ARG, "null plan in request set");
         if (std::find(uniq.begin(), uniq.end(), plans[i]) == uniq.end()) uniq.push_back(plans[i]);
         any_mixed |= plans[i]->precision == CHY_PREC_MIXED;
-        any_blk |= plans[i]->precision == CHY_PREC_FP64_BLKTRI;
+        // with a pivot table every stage schedule is the same launch (blk_warps >= 4
+        // is what its columns fit at most, one CTA per SM)
+        any_blk |= plans[i]->precision == CHY_PREC_FP64_BLKTRI && !plans[i]->t.blk.tab;
         max_batch = std::max(max_batch, plans[i]->max_batch);
     }
     cudaStream_t s = (cudaStream_t)stream;

@@ -175,9 +175,9 @@ int chy_solve_multi(int n, chy_plan *const *plans, const double *const *rho, dou
  *                holding two items per SM.  Both kernels give the same bits;
  *   blk_warps,   the BLKTRI-order path's stage schedule: warps per CTA (the
  *   blk_ctas_per_sm  cyclic-reduction tasks of a stage in flight at once) and
- *                CTAs per SM.  Plans with a pivot table run up to blk_warps
- *                warps (as many as its columns fit, at most 4) on one CTA per
- *                SM.
+ *                CTAs per SM.  Plans with a pivot table run as many warps as
+ *                its columns fit (at most 4) on one CTA per SM whatever the
+ *                schedule, and are left out of this search.
  * Search: from the default schedule, each knob in turn (coordinate descent),
  * `repeats` timed calls per candidate after one warm-up call, CUDA events on
  * `stream`.  The call synchronises `stream`; make it before any capture.  The
