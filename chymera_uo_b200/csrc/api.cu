@@ -1221,8 +1221,7 @@ extern "C" int chy_solve_static(chy_plan *p, const double *rho, double *phi, voi
     // the plan's per-solve arrays, 256-byte aligned pieces, carved from the static array
     const Work &pw = p->w;
     auto al = [](size_t n) { return (n + 31) & ~(size_t)31; };
-    const size_t need = al(pw.sX) + 2 * al(pw.sW) + al(pw.smom) + al(pw.ssub) + al(pw.sscan) +
-                        al(pw.sphac) + al(pw.sdiag);
+    const size_t need = al(pw.sX) + al(pw.sW) + al(pw.smom) + al(pw.ssub) + al(pw.sscan) + al(pw.sphac) + al(pw.sdiag);
     if (need * sizeof(double) > kStaticScratchBytes)
         return fail(CHY_ERR_CAPACITY, "chy_solve_static: this grid needs " + std::to_string(need * sizeof(double)) +
                                           " bytes of work space; the static scratch holds " +

@@ -380,8 +380,8 @@ long long chy_plan_launch_count(const chy_plan *p);
  * for example a simulation that reserves the rest of the GPU for its own
  * arrays, or a time-step loop that must not call the allocator.
  * Its per-solve work space is one static 8 MiB device array per device:
- * enough for the FP64 work space of a 64 x 32 x 64 grid (3.5 MiB, the
- * reference's CPU-run size) or 64 x 32 x 128 (6.5 MiB).  Grids that need more
+ * enough for the FP64 work space of a 64 x 32 x 64 grid (2.5 MiB, the
+ * reference's CPU-run size) up to 112 x 32 x 128 (7.9 MiB).  Grids that need more
  * return CHY_ERR_CAPACITY (chy_last_error gives the size); mixed plans return
  * CHY_ERR_UNSUPPORTED.  The array is cleared (cudaMemsetAsync) at the
  * start of every call.  The first call on each device looks the array up
