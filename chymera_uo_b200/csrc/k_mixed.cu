@@ -86,7 +86,7 @@ struct MixedDev {
                                 // d_k CN_k / d_(k+1) (D = diag(d) symmetrises T_z)
     const float *sw_mul;        // [N+1][ntile][128] multipliers e or f of the radial sweeps
     const float *sw_piv;        // [N+1][ntile][128] pivot reciprocals 1/D
-    double *xbuf;               // [nb][L][K][J] FP64 iterate
+    double *xbuf;               // [nb][L][K][J] FP64 iterate (wide: WideDev::xit)
     size_t sxb;
     double *corr;               // [nb][L][8][2] per mode (wide: per mode and tile): sum delta^2, sum x^2
     size_t scorr;
@@ -103,7 +103,7 @@ struct WideDev {
     float *W;                   // [item][64 nt][128]: products U r, swept in place to w
     size_t sw;
     float *F;                   // [item][KMAX-1][J]: the first solution, x0 = F / d_k
-    double *xit;                // [item][KMAX-1][J] FP64 iterate (two or more corrections)
+    double *xit;                // [item][KMAX-1][J] FP64 iterate (two or more corrections: xbuf)
     size_t sx;
     int nt;
 };
@@ -2897,7 +2897,6 @@ size_t chy_mixed_work_doubles(const chy_plan *p)
         const size_t items = (size_t)hp.L * p->max_batch, Jt = (size_t)round64(hp.J);
         n += al32(items * Jt * 128 / 2);                 // W (FP32)
         n += al32(items * hp.NZ * hp.J / 2 + 1);         // F (FP32)
-        n += al32(items * hp.NZ * hp.J);                 // FP64 iterate
     }
     return n;
 }
@@ -2924,8 +2923,6 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
         wd.W = reinterpret_cast<float *>(q);
         q += al32(items * wd.sw / 2);
         wd.F = reinterpret_cast<float *>(q);
-        q += al32(items * wd.sx / 2 + 1);
-        wd.xit = q;
     }
     if (p->precision == CHY_PREC_MIXED) {
         cudaMallocHost(&p->mx->h_corr, sizeof(double) * d.scorr * p->max_batch);
@@ -2978,6 +2975,7 @@ static int wide_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
     MixedDev x = p->mx->dev;
     x.probe_polls = p->mx->probe_polls;
     const int nit = std::min(1 + p->refine, 8), items = nb * t.L, tiles = items * d.nt;
+    if (nit > 2 && !d.xit) return CHY_ERR_NOT_SETUP;
     for (int it = 0; it < nit; ++it) {
         const bool last = it == nit - 1;
         int st = it == 0   ? wide_launch(k_wide_down<0>, p, tiles, s)
@@ -3132,16 +3130,17 @@ size_t chy_mixed_iterate_bytes(const chy_plan *p) { return p->mx ? p->mx->xbuf_b
 
 int chy_mixed_ensure_iterate(chy_plan *p)
 {
-    // the wide pipeline keeps its own FP64 iterate for any number of corrections
-    if (p->precision != CHY_PREC_MIXED || !p->mx || p->mx->dev.xbuf || p->mx->is_wide) return CHY_OK;
+    if (p->precision != CHY_PREC_MIXED || !p->mx || p->mx->dev.xbuf) return CHY_OK;
     MixedDev &d = p->mx->dev;
-    const size_t bytes = d.sxb * p->max_batch * sizeof(double);
+    const size_t per = p->mx->is_wide ? (size_t)p->hp.L * p->mx->wide.sx : d.sxb;
+    const size_t bytes = per * p->max_batch * sizeof(double);
     if (cudaMalloc(&d.xbuf, bytes) != cudaSuccess) {
         cudaGetLastError();
         d.xbuf = nullptr;
         return CHY_ERR_NOMEM;
     }
     p->mx->xbuf_bytes = bytes;
+    p->mx->wide.xit = d.xbuf;
     // columns >= M and rows >= NZ are read as zeros and never written
     return cudaMemset(d.xbuf, 0, bytes) == cudaSuccess ? CHY_OK : CHY_ERR_CUDA;
 }
