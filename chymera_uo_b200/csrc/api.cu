@@ -339,8 +339,7 @@ int chy_plan_create_limited(const chy_grid *g, int precision, int max_batch, lon
         double *rec = (double *)(D + o_dev), *mul = rec + nth;
         t.th_rec = rec;
         t.th_mul = mul;
-        ce = launch_thomas_table(t, rec, mul, cudaStreamLegacy);
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(cudaStreamLegacy);
+        ce = launch_thomas_table(t, rec, mul, cudaStreamLegacy);   // waited for at the end
         if (ce != cudaSuccess) {
             chy_plan_destroy(p);
             return cuda_fail(ce, "elimination table");
@@ -409,6 +408,8 @@ int chy_plan_create_limited(const chy_grid *g, int precision, int max_batch, lon
         }
     }
     CHY_CUDA(cudaMallocHost(&p->h_diag, sizeof(double) * (kDiagPart * max_batch + 1)));
+    // the table kernels and the cleared work space, for solves on any stream
+    CHY_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     *out = p;
     return CHY_OK;
 }

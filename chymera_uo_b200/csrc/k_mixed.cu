@@ -3141,8 +3141,10 @@ int chy_mixed_ensure_iterate(chy_plan *p)
     }
     p->mx->xbuf_bytes = bytes;
     p->mx->wide.xit = d.xbuf;
-    // columns >= M and rows >= NZ are read as zeros and never written
-    return cudaMemset(d.xbuf, 0, bytes) == cudaSuccess ? CHY_OK : CHY_ERR_CUDA;
+    // columns >= M and rows >= NZ are read as zeros and never written; the solves
+    // may run on any stream
+    return cudaMemset(d.xbuf, 0, bytes) == cudaSuccess && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? CHY_OK
+                                                                                                                : CHY_ERR_CUDA;
 }
 
 void chy_mixed_release(chy_plan *p)
