@@ -152,6 +152,8 @@ def lib():
         L.chy_dbg_mixed_probe.restype = i
         L.chy_dbg_sweep_probe.argtypes = [vp, i]
         L.chy_dbg_sweep_probe.restype = i
+        L.chy_dbg_route.argtypes = [vp]
+        L.chy_dbg_route.restype = i
         L.chy_dbg_blk_redone.argtypes = []
         L.chy_dbg_blk_redone.restype = ll
         L.chy_dbg_mixed_kernel.argtypes = [vp]

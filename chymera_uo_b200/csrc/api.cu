@@ -685,7 +685,7 @@ static int run_batch(chy_plan *p, const BatchPtrs &bp, int nb, cudaStream_t s, b
     CHY_CUDA(mark(3));
     int nl = 0;
     if (p->precision == CHY_PREC_FP64) {
-        CHY_CUDA(launch_solve_fp64(t, p->w, nb, p->num_sms, s));
+        CHY_CUDA(launch_solve_fp64(t, p->w, nb, p->num_sms, s, &p->sweep_on_chip));
         nl = 3;
     } else if (p->precision == CHY_PREC_FP64_BLKTRI) {
         CHY_CUDA(launch_solve_blk(t, p->w, nb, p->num_sms, p->blk_warps, p->blk_ctas_per_sm, s, &nl));
@@ -1269,7 +1269,7 @@ extern "C" int chy_solve_static(chy_plan *p, const double *rho, double *phi, voi
     CHY_CUDA(launch_forward(t, bp, w, 1, s));
     CHY_CUDA(launch_bdy_sums(t, w, 1, s));
     CHY_CUDA(launch_bdy_synth(t, w, 1, s));
-    CHY_CUDA(launch_solve_fp64(t, w, 1, p->num_sms, s));
+    CHY_CUDA(launch_solve_fp64(t, w, 1, p->num_sms, s, &p->sweep_on_chip));
     int nv = 0;
     CHY_CUDA(launch_inverse(t, bp, w, StarDev{}, 1, s, &nv));   // POT3 alone
     p->launches += 1 + 2 + 1 + 3 + nv;
@@ -1281,6 +1281,12 @@ extern "C" long long chy_dbg_blk_redone(void)
     unsigned n = 0;
     const cudaError_t e = blk_redone(&n);
     return e == cudaSuccess ? (long long)n : -cuda_fail(e, "chy_dbg_blk_redone");
+}
+
+extern "C" int chy_dbg_route(const chy_plan *p)
+{
+    if (!p) return -CHY_ERR_ARG;
+    return (p->sweep_on_chip ? 1 : 0) | (p->w.pdl ? 2 : 0);
 }
 
 extern "C" int chy_dbg_sweep_probe(chy_plan *p, int polls)

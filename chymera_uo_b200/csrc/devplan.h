@@ -161,7 +161,8 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 cudaError_t launch_forward(const DevTables &t, const BatchPtrs &bp, const Work &w, int nb, cudaStream_t s);
 cudaError_t launch_bdy_sums(const DevTables &t, const Work &w, int nb, cudaStream_t s);
 cudaError_t launch_bdy_synth(const DevTables &t, const Work &w, int nb, cudaStream_t s);
-cudaError_t launch_solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s);
+// on_chip: the sweeps ran with their rows in tensor memory.
+cudaError_t launch_solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s, bool *on_chip);
 // Doubles of each plane of the FP64 path's elimination table, and its kernel.
 size_t thomas_table_doubles(int J, int K, int L);
 cudaError_t launch_thomas_table(const DevTables &t, double *rec, double *mul, cudaStream_t s);

@@ -2984,6 +2984,7 @@ static int wide_solve(chy_plan *p, int nb, cudaStream_t s, int *launches)
         if (st != CHY_OK) return st;
         cudaError_t e = cudaSuccess;
         // rows in tensor memory while its 512 columns hold them (measured above)
+        p->sweep_on_chip = t.M <= 512;
         if (t.M <= 512) {
             e = ensure_smem((const void *)k_wide_sweep_tm, SwSmem::bytes);
             if (e == cudaSuccess)

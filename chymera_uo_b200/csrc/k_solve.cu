@@ -567,13 +567,13 @@ cudaError_t launch_thomas_table(const DevTables &t, double *rec, double *mul, cu
 }
 
 template <int KP, int MT>
-static cudaError_t solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s)
+static cudaError_t solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s, bool *tm)
 {
     using Z = ZTile<KP, MT>;
     const int items = nb * t.L * ((t.M + Z::JT - 1) / Z::JT);   // at most 64 x 1024 x 512
     // narrower tiles while the items do not fill the SMs twice
     if constexpr (MT > 1)
-        if (items < 2 * num_sms) return solve_fp64<KP, MT / 2>(t, w, nb, num_sms, s);
+        if (items < 2 * num_sms) return solve_fp64<KP, MT / 2>(t, w, nb, num_sms, s, tm);
     cudaError_t e = ensure_smem((const void *)k_zfwd_f64<KP, MT>, Z::kFwdBytes);
     if (e == cudaSuccess) e = ensure_smem((const void *)k_zinv_f64<KP, MT>, Z::kInvBytes);
     auto sweep = KP == 16 && t.K < 16 ? k_thomas_f64<0> : k_thomas_f64<KP>;
@@ -599,6 +599,7 @@ static cudaError_t solve_fp64(const DevTables &t, const Work &w, int nb, int num
             if (e == cudaSuccess)
                 e = launch_pdl(w.pdl, k_thomas_tm<KP>, dim3(groups < num_sms ? groups : num_sms), dim3(128), kTmBytes, s, t, w, groups);
         }
+    *tm = on_chip;
     // k_thomas_f64 never starts early, and hands over at its end: beside a product's
     // 200 KB of shared memory its streaming loads have next to no L1.  Solves one
     // after the other in a graph, both overlapped / so (us): 512x32x64 197 / 91,
@@ -610,12 +611,12 @@ static cudaError_t solve_fp64(const DevTables &t, const Work &w, int nb, int num
     return launch_pdl(w.pdl, k_zinv_f64<KP, MT>, dim3(grid), dim3(kZThreads), Z::kInvBytes, s, t, w, nb);
 }
 
-cudaError_t launch_solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s)
+cudaError_t launch_solve_fp64(const DevTables &t, const Work &w, int nb, int num_sms, cudaStream_t s, bool *on_chip)
 {
-    if (t.K <= 16) return solve_fp64<16, 4>(t, w, nb, num_sms, s);
-    if (t.K <= 32) return solve_fp64<32, 8>(t, w, nb, num_sms, s);
-    if (t.K <= 64) return solve_fp64<64, 8>(t, w, nb, num_sms, s);
-    if (t.K <= 128) return solve_fp64<128, 8>(t, w, nb, num_sms, s);
+    if (t.K <= 16) return solve_fp64<16, 4>(t, w, nb, num_sms, s, on_chip);
+    if (t.K <= 32) return solve_fp64<32, 8>(t, w, nb, num_sms, s, on_chip);
+    if (t.K <= 64) return solve_fp64<64, 8>(t, w, nb, num_sms, s, on_chip);
+    if (t.K <= 128) return solve_fp64<128, 8>(t, w, nb, num_sms, s, on_chip);
     return cudaErrorInvalidValue;
 }
 

@@ -56,6 +56,7 @@ struct chy_plan {
     chy::StarDev star;             // ExternalPot (chy_plan_set_external, chy_plan_set_binary)
     double bin_a = 0.0;            // the BINARY companion's separation ABIN
     int last_slot = 0;             // batch slot of the latest solve launched
+    bool sweep_on_chip = false;    // its radial sweeps kept their rows in tensor memory
     bool profile = false;
     // One event set per profiled launch sequence, read back lazily (after
     // the caller has synchronised) so profiling adds no host waits.

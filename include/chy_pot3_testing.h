@@ -59,6 +59,11 @@ int chy_dbg_mixed_probe(chy_plan *p, int polls);
  * become NaN and the solve reports CHY_ERR_TIMEOUT.  0 switches it off. */
 int chy_dbg_sweep_probe(chy_plan *p, int polls);
 
+/* How the plan's last solve was launched: bit 0, its radial sweeps ran with their
+ * rows in tensor memory (FP64 plans, wide mixed pipeline); bit 1, its launches
+ * overlapped.  -CHY_ERR_ARG for a null plan. */
+int chy_dbg_route(const chy_plan *p);
+
 /* PRDCT passes of BLKTRI-order solves on the current device so far that the
  * tabulated pivots did not settle and that were formed again with divisions;
  * waits for the device. */
