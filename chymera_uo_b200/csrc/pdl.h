@@ -24,13 +24,28 @@
 // 447, but 495 waited for).
 //
 // Waiting CTAs hold registers and shared memory, and a kernel that starts beside
-// one with much shared memory keeps that one's small L1.  So launches overlap
-// (Work::pdl) in a solve that has the device to itself and is short: up to
-// kPdlCells cells in the launch sequence.  Measured with and without: one solve of
-// 64x32x64 FP64 59.4 -> 43.2 us, mixed 61.1 -> 58.8, of 256x128x256 mixed 250.7
-// -> 246.7; but eight solves of 256x128x256 FP64 2.20 -> 2.35 ms, four of
-// 512x128x512 5.28 -> 5.41, 24 grids on eight streams 1.59 -> 1.61, and a time
-// step whose star and source kernels overlapped too 429 -> 470 us.
+// one with much shared memory keeps that one's small L1 (which is why k_thomas_f64
+// and the kernels around it take turns, k_solve.cu).  So launches overlap
+// (Work::pdl) in a launch sequence of up to kPdlCells cells that this library runs
+// by itself: not beside others of chy_solve_multi, nor in the server.  A caller's
+// own streams are not known here; two plans on two streams take the same or less
+// time for it (mixed 128x64x128 113 -> 107 us a pair, FP64 114 -> 102, BLKTRI 2.08 ->
+// 2.07 ms).  Measured without -> with, us, solves one after the other in a graph, and
+// one at a time waited for by the host:
+//   0.14 M cells  FP64 64x32x64      39.7 -> 38.2    79.8 -> 63.0
+//                 mixed              49.4 -> 47.6    75.8 -> 63.0
+//   4.2 M         FP64 128x64x128 x4  155 -> 154      196 -> 180
+//   8.2 M         FP64 256x128x256    320 -> 317      354 -> 337
+//                 mixed               242 -> 243      270 -> 264
+//                 FP64 512x64x256     300 -> 297      334 -> 318
+//                 mixed               450 -> 448      492 -> 469
+//   8.8 M         mixed 64x32x64 x64  777 -> 774      895 -> 890
+//   16.4 M        FP64 256x128x256 x2 576 -> 574      613 -> 597
+//                 mixed               424 -> 432      455 -> 455
+//   33 M          mixed 256x128x256 x4 738 -> 750     774 -> 777
+//   66 M          FP64 256x128x256 x8 2042 -> 2055   2092 -> 2091
+//                 mixed              1413 -> 1444    1460 -> 1480
+// The line lies between 8.8 M and the first sizes that lose.
 #pragma once
 
 #include <cuda_runtime.h>
