@@ -15,7 +15,8 @@
 // spread over its warps, with a barrier between stages.  k_blk_solve_tab reads
 // the plan's table of pivots; k_blk_solve divides, keeps its elimination
 // multipliers D and partial solution W in per-warp scratch in global memory, and
-// serves plans without a table (more than 384 rows, or little free memory).
+// serves plans without a table (fewer than 17 or more than 408 rows, no memory for
+// one, or the caller's limit).
 //
 // This file is compiled with --fmad=false and its quotients are the IEEE ones:
 // every product, sum and quotient rounds as the reference's, so the modes equal
@@ -257,8 +258,9 @@ __global__ void __launch_bounds__(NW * 32) k_blk_solve(DevTables t, Work w, int 
 // formed again with divisions.  (Solutions of columns without density decay over
 // the rows, to 1e-155 at JMAX = 256: a threshold of 2^-500 redid one pass in ten.)
 // One solve of 64x32x64 / 256x128x256: 2.29 / 50.5 ms with two divisions a row
-// and the vectors in L2, 0.585 / 8.8 ms now, 113 cycles a row of both sweeps
-// (their dependent chains are 48); a batch of 32 of the latter 74.3 -> 59.2 ms.
+// and the vectors in L2, 0.563 / 8.8 ms now, 112 cycles a row of both sweeps
+// (clock64 around the sweeps: elimination 64, substitution 48; their dependent chains
+// are 32 and 16); a batch of 32 of the latter 74.3 -> 59.2 ms.
 // ---------------------------------------------------------------------------
 constexpr double kBlkDenMin = 0x1p-100, kBlkDenMax = 0x1p100, kBlkNumMin = 0x1p-860;
 
