@@ -600,13 +600,17 @@ static cudaError_t solve_fp64(const DevTables &t, const Work &w, int nb, int num
                 e = launch_pdl(w.pdl, k_thomas_tm<KP>, dim3(groups < num_sms ? groups : num_sms), dim3(128), kTmBytes, s, t, w, groups);
         }
     *tm = on_chip;
-    // k_thomas_f64 never starts early, and hands over at its end: beside a product's
-    // 200 KB of shared memory its streaming loads have next to no L1.  Solves one
-    // after the other in a graph, both overlapped / so (us): 512x32x64 197 / 91,
-    // 300x128x64 217 / 176, 512x64x256 452 / 296, 128x64x128 x4 175 / 154, 64x32x64
-    // x32 219 / 214; with only its own early start left 91, 199, 416, 175, 218.
-    if (!on_chip)
-        e = launch_pdl(false, sweep, dim3((t.L + mpb - 1) / mpb, nb), dim3(128), (size_t)t.M * sizeof(double), s, t, w);
+    // k_thomas_f64 hands over at its end and starts early in up to sixteen CTAs only:
+    // beside a product's 200 KB of shared memory its streaming loads have next to no
+    // L1.  Queued solves, both kernels overlapped from their start / so (us): 512x32x64
+    // 202 / 104, 300x128x64 221 / 181, 512x64x128 322 / 205, 512x128x128 490 / 380,
+    // 129x16x64 57 / 52.  Early start against none: 4 CTAs (257x16x32) 61 / 64, 8
+    // (512x16x64) 94 / 95, 16 (257x16x128) 81 / 82, 32 (300x32x128) 98 / 94, 64
+    // (300x64x128) 171 / 144, 128 (512x128x128) 530 / 380.
+    if (!on_chip) {
+        const dim3 g((t.L + mpb - 1) / mpb, nb);
+        e = launch_pdl(w.pdl && g.x * g.y <= 16, sweep, g, dim3(128), (size_t)t.M * sizeof(double), s, t, w);
+    }
     if (e != cudaSuccess) return e;
     return launch_pdl(w.pdl, k_zinv_f64<KP, MT>, dim3(grid), dim3(kZThreads), Z::kInvBytes, s, t, w, nb);
 }
