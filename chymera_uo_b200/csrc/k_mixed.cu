@@ -92,6 +92,7 @@ struct MixedDev {
     size_t scorr;
     int *err;                   // error word
     int nit;                    // approximate solves (1 + corrections)
+    int lim0;                   // half_limit for TMASS just below one
     int ntile;                  // MMA N = J rounded up to 64 (<= 256)
     int probe_polls;            // test hook: > 0 makes every CTA first wait this many
                                 // polls on a barrier nothing arrives on (0: off)
@@ -373,21 +374,27 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// power-of-two scale that maps max|v| below 2^14
-__device__ __forceinline__ float pow2_scale(float vmax)
+// exponent k of the power-of-two scale that maps max|v| = vmax below 2^14, but at
+// most lim: 126 keeps the scale and its reciprocal in single precision (what is
+// smaller than 2^-112 goes through the product with fewer bits)
+__device__ __forceinline__ int pow2_exp(float vmax, int lim = 126)
 {
-    if (!(vmax > 0.0f) || !isfinite(vmax)) return 1.0f;
-    int e;
-    frexpf(vmax, &e);
-    return ldexpf(1.0f, 14 - e);
+    const int e = __float_as_int(vmax) >> 23;   // vmax >= 0: the biased exponent
+    return vmax == 0.0f || e >= 255 ? 0 : min(140 - e, lim);
 }
-// its exponent k: pow2_scale(vmax) = 2^k
-__device__ __forceinline__ int pow2_exp(float vmax)
+__device__ __forceinline__ float pow2_scale(float vmax) { return ldexpf(1.0f, pow2_exp(vmax)); }
+
+// Largest scale exponent of a radial half in the fused kernels' sweeps.  A half's
+// scale comes from its own residual, but its rows then hold the other half's
+// solution too: where the residual is next to nothing (the tail of a body without a
+// density floor, in a mode without a boundary value) that would leave single
+// precision.  So a residual far below the mean of the solve's right-hand side, 4 pi G
+// TMASS over the grid's volume, is scaled as if it were 2^-gap of it (mixed_lim0).
+__device__ __forceinline__ int half_limit(const DevTables &t, const Work &w, const MixedDev &x, int b)
 {
-    if (!(vmax > 0.0f) || !isfinite(vmax)) return 0;
-    int e;
-    frexpf(vmax, &e);
-    return 14 - e;
+    const double tmass = __ldcg(w.scan + (size_t)b * w.sscan + (size_t)t.nsub * 2 * t.ncol);
+    const int e = ((__double2hiint(tmass) >> 20) & 0x7ff) - 1022;   // |TMASS| < 2^e
+    return min(x.lim0 - e, 126);
 }
 
 // Writes the FP16 hi/lo split of v (already scaled) for element (row, k).
@@ -911,7 +918,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_mixed(DevTables t, Work w, Mixe
             rmax0 = f_red[0];
             rmax1 = f_red[8];
             for (int i = 1; i < 8; ++i) { rmax0 = fmaxf(rmax0, f_red[i]); rmax1 = fmaxf(rmax1, f_red[8 + i]); }
-            const int k1h0 = pow2_exp(rmax0), k1h1 = pow2_exp(rmax1);
+            const int lim = half_limit(t, w, x, b), k1h0 = pow2_exp(rmax0, lim), k1h1 = pow2_exp(rmax1, lim);
             const float s1 = ldexpf(1.0f, jh ? k1h1 : k1h0);   // this thread splits half jh
             // ---- TMEM r -> B tile (row j, K index k), FP16 hi/lo
             for (int c0 = jh * NH; c0 < (jh + 1) * NH; c0 += 32) {
@@ -1497,6 +1504,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_pair(DevTables t, Work w, Mixed
         }
         double *cr = x.corr + (size_t)b * x.scorr + (size_t)l * 16 + 8 * rank;
         const int row0 = (b * t.L + l) * K;             // first tensor-map row of this item
+        const int lim = half_limit(t, w, x, b);
         double u0 = 0.0;                                // scale of x0 in tensor memory (2^eu0)
         int eu0 = 0;
         double ym_keep = 0.0, edge_in = 0.0;            // X(k, M); the peer's x0 edge in u0 units
@@ -1660,7 +1668,7 @@ __global__ void __launch_bounds__(256, 1) k_mode_pair(DevTables t, Work w, Mixed
                 if (gt == 0) mbar_arrive(bar_stagger);
                 stag_sent = true;
             }
-            const int k1 = pow2_exp(group_max(rmax));
+            const int k1 = pow2_exp(group_max(rmax), lim);
             if (s_flag[g]) { failed = true; break; }
             const float s1 = ldexpf(1.0f, k1);
             // ---- TMEM r -> B tile (row j, K index k), FP16 hi/lo
@@ -2321,7 +2329,7 @@ __global__ void __launch_bounds__(256, 2) k_wide_down(DevTables t, Work w, Mixed
         if constexpr (kSrc == 1)
             if (more) load_f(tile + gridDim.x);
         float *dst = d.W + (size_t)item * d.sw + (size_t)(j0 + 32 * (warp >> 2)) * 128 + 32 * (warp & 3) + lane;
-        const float unscale = 1.0f / (kAScale * s);
+        const float unscale = (1.0f / kAScale) * (1.0f / s);
         float o[32];
         if (ok) tm_ld32(c.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * (warp >> 2), o);
 #pragma unroll
@@ -2392,7 +2400,7 @@ __global__ void __launch_bounds__(256, 2) k_wide_up(DevTables t, Work w, MixedDe
             *reinterpret_cast<uint2 *>(c.sBl + o) = make_uint2(pack_half2(lo[0], lo[1]), pack_half2(lo[2], lo[3]));
         }
         const bool ok = wide_product(c, true);
-        const float unscale = 1.0f / (kAScale * s);
+        const float unscale = (1.0f / kAScale) * (1.0f / s);
         {
             float o[32];
             if (ok) tm_ld32(c.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * (warp >> 2), o);
@@ -2888,6 +2896,21 @@ static size_t corr_stride(const chy::HostPlan *hp)
     return (size_t)hp->L * 16 * (mixed_fused(hp) ? 1 : round64(hp->J) / 64);
 }
 
+// half_limit's constant.  With a residual scaled to 2^14 and the eigenbasis to 2^12, a
+// solution of up to R^2 times the largest right-hand side (itself some 2^17 means in
+// a body of a thousandth of the grid) stays below 2^127 for a gap of 84 bits less R^2's;
+// 64 bits are more than the FP64 sum over the modes keeps.
+static int mixed_lim0(const chy::HostPlan &hp)
+{
+    const double rad = std::fabs(hp.rhf[hp.J]), vol = 3.0 * rad * rad * 2.0 * std::fabs(hp.zhf[hp.K]);
+    const double unit = std::fabs(hp.pig4) / vol;   // the mean right-hand side of TMASS = 1
+    if (!(unit > 0.0) || !std::isfinite(unit)) return 126 + 1024;
+    int e = 0, er = 0;
+    std::frexp(unit, &e);
+    std::frexp(rad * rad, &er);
+    return 14 + std::min(std::max(84 - er, 20), 64) - e;
+}
+
 size_t chy_mixed_work_doubles(const chy_plan *p)
 {
     if (p->precision != CHY_PREC_MIXED) return 0;
@@ -2911,6 +2934,7 @@ void chy_mixed_bind_work(chy_plan *p, double *base)
     d.xbuf = nullptr;
     d.corr = base;
     d.err = p->w.stat;
+    d.lim0 = mixed_lim0(hp);
     d.ntile = round64(hp.J);
     if (p->precision == CHY_PREC_MIXED && !mixed_fused(&hp)) {
         WideDev &wd = p->mx->wide;
