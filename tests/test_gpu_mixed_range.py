@@ -62,3 +62,12 @@ def test_small_densities(chylib, J, K, L):
     for scale, tol in ((1e30, 1e-10), (1e-20, 1e-10), (1e-25, 1e-8), (1e-30, np.inf)):
         e = error(chylib, np.asfortranarray(rho * scale), J, K, L)
         assert np.isfinite(e) and e < tol, (scale, e)
+
+
+@pytest.mark.parametrize("J,K,L", [(127, 32, 32), (128, 32, 32), (257, 16, 32)])
+def test_centimetres_and_grams(chylib, J, K, L):
+    """The same bodies in units in which lengths are 1e13 and the right-hand side 1e-15:
+    the solution is 2^86 times the residual."""
+    for sigma, r0 in ((0.2, 0.0), (0.05, 0.0), (0.05, 0.9), (0.02, 0.0)):
+        e = error(chylib, body(J, K, L, sigma, r0) * 1e-9, J, K, L, rof3n=1e13 / J, zof3n=0.5e13 / K, grav=6.67e-8)
+        assert e < 1e-10, (sigma, r0, e)
